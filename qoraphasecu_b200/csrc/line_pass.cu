@@ -19,8 +19,10 @@
 #include "column_pass.cuh"
 #include "fast_pass.cuh"
 #include "line_pass.cuh"
+#include "mixed_pass.cuh"
 #include "projection.cuh"
 #include "reduce.cuh"
+#include "two_stage_pass.cuh"
 
 namespace qpb {
 
@@ -353,6 +355,7 @@ void configure_line_passes() {
   allow_smem(line_pass_kernel<Mode::kGrad, __nv_bfloat16>);
   configure_fast_passes();
   configure_column_passes();
+  configure_mixed_passes();
 }
 
 int choose_lpc(int L, int S, int lines_per_start) {
@@ -375,6 +378,10 @@ void launch_line_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
     throw std::logic_error("line pass: a line-major tiled amplitude needs the column pass");
   }
   if (fast_passes_enabled() && fast_pass_supports(p)) return launch_fast_pass(mode, p, stream);
+  if (fast_passes_enabled() && two_stage_supports(mode, p)) {
+    return launch_two_stage_pass(mode, p, stream);
+  }
+  if (fast_passes_enabled() && mixed_pass_supports(p)) return launch_mixed_pass(mode, p, stream);
   const bool touches_x = mode == Mode::kFwdFromX || mode == Mode::kUpd || mode == Mode::kBlurMag;
   if (p.wave_half || (touches_x && p.iter_half)) {
     throw std::logic_error("line pass: fp16 storage needs the register-resident or column pass");

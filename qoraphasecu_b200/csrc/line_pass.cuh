@@ -75,6 +75,9 @@ struct PassParams {
   int starts_total;               // error row width
   int stages;
   int radix[kMaxStages];
+  const LinePlan* plan;           // host only: the mixed-radix pass's stages
+  const float2* mixed_twiddle;    // its stage-major table
+  const float2* two_stage_twiddle;  // the two-stage pass's table, or null
   float scale;                    // 1/sqrt(n) (kMod)
   float blur_k;                   // -2 (pi sigma)^2 (kBlur)
   int level_method;               // 0 none, 1 max, 2 rms (kBlur)

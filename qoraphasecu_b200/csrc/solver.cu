@@ -28,6 +28,7 @@
 #include "persistent.cuh"
 #include "resident.cuh"
 #include "solver.hpp"
+#include "two_stage_pass.cuh"
 
 namespace qpb {
 
@@ -224,6 +225,7 @@ PassRunner::PassRunner(Dims3 d, int ndim, PlanCache& plans)
   configure_line_passes();
   for (int a = 0; a < 3; ++a) {
     plans_[a] = (ndim == 2 && a == 0) ? nullptr : &plans.get(axis_len(d, a));
+    if (plans_[a]) configure_two_stage(axis_len(d, a));
   }
 }
 
@@ -241,6 +243,9 @@ PassParams PassRunner::params(Mode mode, int axis3, int batch) const {
   for (int s = 0; s < plan.stages; ++s) p.radix[s] = plan.radix[s];
   p.twiddle = plan.twiddle;
   p.stage_twiddle = plan.stage_twiddle;
+  p.plan = &plan;
+  p.mixed_twiddle = plan.mixed_twiddle;
+  p.two_stage_twiddle = plan.two_stage_twiddle;
   p.scale = 1.0f / std::sqrt(static_cast<float>(p.n));
   p.amp_stride = 0;
   p.starts_per_problem = 1;

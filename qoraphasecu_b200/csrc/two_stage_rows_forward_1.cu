@@ -1,0 +1,9 @@
+// Two-stage passes, mode kFwdFromX along rows: slice 1 of the lengths.
+
+#include "two_stage_kernel.cuh"
+
+namespace qpb {
+
+template TwoStageList two_stage_slice<Mode::kFwdFromX, true, 1>();
+
+}  // namespace qpb
