@@ -3,8 +3,12 @@
 // memory, runs mixed-radix Stockham stages between two shared buffers, applies
 // the fused point-wise step and stores the lines back.
 //
-// This is the path for every shape; power-of-two lengths additionally have the
-// register-resident kernels of fast_pass.cu.
+// Lengths whose prime factors are at most 13 run the register-resident kernels
+// instead (fast_pass.cu and column_pass.cu for powers of two, two_stage_kernel.cuh
+// and mixed_pass_kernel.cuh for the rest); this kernel keeps the lengths with a
+// larger prime factor and the axes of length 1. It is the slower one wherever
+// another runs: an iteration of 16 starts of 240 x 240 took 71 us here and takes
+// 18 us there.
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -378,6 +382,9 @@ void launch_line_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
     throw std::logic_error("line pass: a line-major tiled amplitude needs the column pass");
   }
   if (fast_passes_enabled() && fast_pass_supports(p)) return launch_fast_pass(mode, p, stream);
+  // A length compiled on its own before the run-time radices: 96 x 96 with 4
+  // starts runs an iteration in 6.0 us against 13.7, 480 x 480 with 16 starts
+  // in 53 against 84.
   if (fast_passes_enabled() && two_stage_supports(mode, p)) {
     return launch_two_stage_pass(mode, p, stream);
   }

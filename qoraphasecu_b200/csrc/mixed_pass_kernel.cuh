@@ -1,7 +1,8 @@
 // The mixed-radix line-pass kernel and its launch, instantiated per group of
-// modes by mixed_pass_*.cu. Lines of any length whose prime factors are at
-// most 13 (the lengths 2^k of 16..1024 whose lines fill the tiles of
-// fast_pass.cu or column_pass.cu run there instead).
+// modes by mixed_pass_*.cu: lines of any length whose prime factors are at
+// most 13, radices chosen at run time. Lengths with a kernel of their own
+// (column_pass.cu, fast_pass.cu, two_stage_kernel.cuh) come here only for the
+// modes and line counts those do not take.
 //
 // A line of L = R_0 R_1 .. R_{K-1} points (every radix 2..16, as few stages as
 // the length allows; fft_plan.cpp) is transformed by K Stockham stages. A
@@ -20,6 +21,10 @@
 // writing item (o = (j / N) N R + j mod N + q N) and the reading one (j' + q M',
 // M' a multiple of N R) then step through it by a constant per q, and P keeps
 // the items of a half-warp on different banks.
+//
+// Bound: issue and instruction fetch (the stages of a launch are a few of the
+// many compiled here). Against line_pass.cu, which ran these lengths before:
+// 16 starts of 240 x 240 71 -> 23 us an iteration, 2 starts of 96^3 125 -> 51.
 //
 // Columns (stride S > 1): adjacent lines on adjacent threads and next to each
 // other in shared memory ([slot][line]), so a half-warp reads neighbouring
