@@ -496,7 +496,8 @@ class Solver:
         _lib.check(self._lib.qpb_results_device(
             self._handle, ctypes.c_void_p(objects.data_ptr()),
             ctypes.c_void_p(supports.data_ptr()), _lib.ptr(errors)))
-        return [Reconstruction(objects[s], supports[s].bool(), errors[s]) for s in range(starts)]
+        supports = supports.view(torch.bool)  # the device writes 0 or 1
+        return [Reconstruction(objects[s], supports[s], errors[s]) for s in range(starts)]
 
     def close(self):
         if getattr(self, "_handle", None):

@@ -6,7 +6,9 @@
 
 #include "aux_kernels.cuh"
 #include "common.cuh"
+#include "dependent_launch.cuh"
 #include "reduce.cuh"
+#include "roll.cuh"
 
 namespace qpb {
 
@@ -112,18 +114,45 @@ __global__ void detwin_apply_kernel(std::uint8_t* support, Dims3 d, int axis3,
 }
 
 template <class T>
-__global__ void roll_kernel(const T* in, T* out, Dims3 d, int o0, int o1, int o2) {
-  const long long n = d.n();
-  in += blockIdx.y * n;
-  out += blockIdx.y * n;
-  QPB_FOR(i, n) {
-    const int x = static_cast<int>(i % d.d2);
-    const int y = static_cast<int>((i / d.d2) % d.d1);
-    const int z = static_cast<int>(i / (static_cast<long long>(d.d1) * d.d2));
-    const int sz = (z + o0) % d.d0;
-    const int sy = (y + o1) % d.d1;
-    const int sx = (x + o2) % d.d2;
-    out[i] = in[(static_cast<long long>(sz) * d.d1 + sy) * d.d2 + sx];
+__global__ void roll_kernel(const T* in, T* out, Dims3 d, RollOffsets o) {
+  const long long off = blockIdx.y * d.n();
+  for_rolled(d, o, [&](long long i, long long src, int, int) { out[off + i] = in[off + src]; });
+}
+
+__global__ void roll_cut_kernel(const float2* in, const std::uint8_t* support, float2* out, Dims3 d,
+                                RollOffsets o, const float* peaks, int starts_per_problem) {
+  const long long off = blockIdx.y * d.n();
+  float scale = 1.0f;
+  if (peaks) {
+    const float peak = peaks[blockIdx.y / starts_per_problem];
+    scale = 1.0f / (peak > 0.0f ? peak : 1.0f);
+  }
+  for_rolled(d, o, [&](long long i, long long src, int, int) {
+    float2 v = {0.0f, 0.0f};
+    if (support[off + i]) {
+      v = in[off + src];
+      if (peaks) v = cscale(v, scale);
+    }
+    out[off + i] = v;
+  });
+}
+
+__global__ void roll_results_kernel(const float2* x, const std::uint8_t* support, float2* objects,
+                                    std::uint8_t* supports, Dims3 d, RollOffsets o) {
+  const long long off = blockIdx.y * d.n();
+  for_rolled(d, o, [&](long long i, long long src, int, int) {
+    objects[off + i] = x[off + src];
+    supports[off + i] = support[off + src];
+  });
+}
+
+// A run's control block, its iteration counters and its error rows.
+__global__ void begin_run_kernel(Ctrl* ctrl, Ctrl value, int counters, double* errs,
+                                 long long count) {
+  QPB_FOR(i, count) errs[i] = 0.0;
+  if (blockIdx.x == 0) {
+    for (int c = threadIdx.x; c < counters; c += blockDim.x) value.counters[c] = 0;
+    if (threadIdx.x == 0) *ctrl = value;
   }
 }
 
@@ -146,11 +175,30 @@ __global__ void from_half_kernel(const __half2* in, float2* out, long long count
   QPB_FOR(i, count) { out[i] = __half22float2(in[i]); }
 }
 
+dim3 roll_grid(Dims3 d, int batch) {
+  return {roll_blocks(d, 148 * 16), static_cast<unsigned>(batch), 1};
+}
+
 dim3 grid(long long n, int batch) {
   return {static_cast<unsigned>(blocks_for(n)), static_cast<unsigned>(batch), 1};
 }
 
 }  // namespace
+
+void configure_aux_kernels() {
+  prefer_shared_memory(random_wave_kernel);
+  prefer_shared_memory(support_project_kernel);
+  prefer_shared_memory(threshold_kernel);
+  prefer_shared_memory(detwin_moment_kernel);
+  prefer_shared_memory(detwin_apply_kernel);
+  prefer_shared_memory(roll_kernel<float2>);
+  prefer_shared_memory(roll_kernel<std::uint8_t>);
+  prefer_shared_memory(roll_cut_kernel);
+  prefer_shared_memory(roll_results_kernel);
+  prefer_shared_memory(begin_run_kernel);
+  prefer_shared_memory(set_coefficients_kernel);
+  prefer_shared_memory(set_ctrl_kernel);
+}
 
 void random_wave(float2* w, const float* amplitude, long long amp_stride, int starts_per_problem,
                  long long n, int batch, std::uint64_t seed, std::uint64_t first_start,
@@ -191,9 +239,31 @@ void detwin(std::uint8_t* support, unsigned long long* moments, Dims3 d, int axi
 
 template <class T>
 void roll(const T* in, T* out, Dims3 d, int batch, bool to_fft_order, cudaStream_t stream) {
-  auto off = [&](int len) { return to_fft_order ? len / 2 : len - len / 2; };
-  roll_kernel<T><<<grid(d.n(), batch), kThreads, 0, stream>>>(in, out, d, off(d.d0), off(d.d1),
-                                                              off(d.d2));
+  roll_kernel<T><<<roll_grid(d, batch), roll_block(d), 0, stream>>>(
+      in, out, d, roll_offsets(d, to_fft_order));
+  QPB_CHECK(cudaGetLastError());
+  count_launches(1);
+}
+
+void roll_cut(const float2* in, const std::uint8_t* support, float2* out, Dims3 d, int batch,
+              const float* peaks, int starts_per_problem, cudaStream_t stream) {
+  roll_cut_kernel<<<roll_grid(d, batch), roll_block(d), 0, stream>>>(
+      in, support, out, d, roll_offsets(d, true), peaks, starts_per_problem);
+  QPB_CHECK(cudaGetLastError());
+  count_launches(1);
+}
+
+void roll_results(const float2* x, const std::uint8_t* support, float2* objects,
+                  std::uint8_t* supports, Dims3 d, int batch, cudaStream_t stream) {
+  roll_results_kernel<<<roll_grid(d, batch), roll_block(d), 0, stream>>>(
+      x, support, objects, supports, d, roll_offsets(d, false));
+  QPB_CHECK(cudaGetLastError());
+  count_launches(1);
+}
+
+void begin_run(Ctrl* ctrl, const Ctrl& value, int counters, double* errs, long long count,
+               cudaStream_t stream) {
+  begin_run_kernel<<<blocks_for(count), kThreads, 0, stream>>>(ctrl, value, counters, errs, count);
   QPB_CHECK(cudaGetLastError());
   count_launches(1);
 }

@@ -40,6 +40,21 @@ void detwin(std::uint8_t* support, unsigned long long* moments, Dims3 d, int axi
 template <class T>
 void roll(const T* in, T* out, Dims3 d, int batch, bool to_fft_order, cudaStream_t stream);
 
+// Given starts: out[b] = in[b] rolled to FFT order, 0 outside support[b],
+// divided by peaks[b / starts_per_problem] where peaks is not null (0 counts
+// as 1).
+void roll_cut(const float2* in, const std::uint8_t* support, float2* out, Dims3 d, int batch,
+              const float* peaks, int starts_per_problem, cudaStream_t stream);
+
+// objects[b] = x[b] and supports[b] = support[b], both rolled to centre origin.
+void roll_results(const float2* x, const std::uint8_t* support, float2* objects,
+                  std::uint8_t* supports, Dims3 d, int batch, cudaStream_t stream);
+
+// Writes the whole control block and zeroes its `counters` iteration counters
+// and the `count` error numerators at `errs`.
+void begin_run(Ctrl* ctrl, const Ctrl& value, int counters, double* errs, long long count,
+               cudaStream_t stream);
+
 // Writes the control block fields of a stage.
 void set_coefficients(Ctrl* ctrl, float a, float b, cudaStream_t stream);
 
@@ -54,5 +69,9 @@ void scale_complex(float2* x, long long count, float scale, cudaStream_t stream)
 // elements, for the fp16 iterate of the half variant.
 void to_half(const float2* in, void* out, long long count, cudaStream_t stream);
 void from_half(const void* in, float2* out, long long count, cudaStream_t stream);
+
+// Gives the kernels that run between a solver's passes the passes' carve-out
+// (prefer_shared_memory); once per device, outside stream capture.
+void configure_aux_kernels();
 
 }  // namespace qpb

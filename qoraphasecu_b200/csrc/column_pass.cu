@@ -17,7 +17,6 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
-#include <set>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -217,6 +216,11 @@ void launch_length(Mode mode, const PassParams& p, cudaStream_t stream) {
 template <int L, Mode M, class AmpT, class WT, int LINES>
 void allow_lines() {
   constexpr int bytes = ColumnStaging<L, M, AmpT, WT, LINES>::kBytes;
+  prefer_shared_memory(
+      column_pass_kernel<L, M, AmpT, WT, LINES, ColumnTiling<L, WT, LINES>::MIN_CTAS>);
+  if constexpr (kHasWide<L, M, WT>) {
+    prefer_shared_memory(column_pass_kernel<L, M, AmpT, WT, LINES, kWideCtas>);
+  }
   if constexpr (bytes > 48 * 1024) {
     QPB_CHECK(cudaFuncSetAttribute(
         column_pass_kernel<L, M, AmpT, WT, LINES, ColumnTiling<L, WT, LINES>::MIN_CTAS>,
@@ -299,17 +303,14 @@ void launch_column_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
   }
 }
 
-void configure_column_passes() {
-  static std::mutex mutex;
-  static std::set<int> done;
-  int device = 0;
-  QPB_CHECK(cudaGetDevice(&device));
-  std::lock_guard<std::mutex> lock(mutex);
-  if (!done.insert(device).second) return;
-  allow_length<64>();
-  allow_length<128>();
-  allow_length<256>();
-  allow_length<512>();
+void configure_column_pass(int L) {
+  switch (L) {
+    case 64: return allow_length<64>();
+    case 128: return allow_length<128>();
+    case 256: return allow_length<256>();
+    case 512: return allow_length<512>();
+    default: return;
+  }
 }
 
 }  // namespace qpb

@@ -35,8 +35,8 @@ void launch_column_pass(Mode mode, const PassParams& p, cudaStream_t stream);
 // p.w as {S, L, p.lines / S} elements, box [1][L][8], 64-byte swizzle.
 CUtensorMap column_wave_map(const PassParams& p);
 
-// Raises the dynamic shared-memory limit where needed; once per device,
-// outside stream capture.
-void configure_column_passes();
+// Sets the shared-memory attributes of the kernels for columns of L points on
+// the current device (configure_line_passes).
+void configure_column_pass(int L);
 
 }  // namespace qpb

@@ -1,4 +1,5 @@
-// Programmatic dependent launch of the streamed line passes.
+// Programmatic dependent launch of the streamed line passes, and the launch
+// attribute their kernels share.
 //
 // A pass is launched with cudaLaunchAttributeProgrammaticStreamSerialization,
 // which lets its CTAs start while the kernel before it in the stream (the
@@ -47,6 +48,17 @@ void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, std::siz
   config.attrs = &attr;
   config.numAttrs = 1;
   QPB_CHECK(cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...));
+}
+
+// Gives `kernel` the SM's largest shared-memory carve-out. Left to itself the
+// driver picks a carve-out per kernel from what its blocks need, and where two
+// passes that follow each other get different ones every change drains the
+// SMs: an iteration of 4 starts of 256 x 256 (135 KB of modulus blocks per SM,
+// 219 KB of update blocks) took 11.1 us, with one carve-out 8.8.
+template <class... Params>
+void prefer_shared_memory(void (*kernel)(Params...)) {
+  QPB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared));
 }
 
 }  // namespace qpb

@@ -14,8 +14,11 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
+#include "dependent_launch.cuh"
 #include "device_setup.cuh"
+#include "roll.cuh"
 #include "solver.hpp"
 
 namespace qpb {
@@ -79,27 +82,28 @@ __global__ void threshold_kernel(const float* mag, long long n, const unsigned* 
   QPB_LOOP(i, n) out[i] = mag[i] > level;
 }
 
-// Element e (FFT order) of one problem goes to index `tiled(e)` of the
-// signed-amplitude array: the modulus pass's CTA order for columns, element j
-// of line c of CTA tile t at (t * L + j) * lines + c (element-major, the
+// Where element `row` d2 + x (FFT order) of one problem goes in the signed-
+// amplitude array: the modulus pass's CTA order for columns, element j of line
+// c of CTA tile t at (t * L + j) * lines + c (element-major, the
 // register-resident pass) or at (t * lines + c) * L + (j + r_c) mod L
 // (line-major, the TMA column pass, r_c = amp_line_rotation(L, c)); FFT order
-// otherwise.
-__device__ __forceinline__ long long tiled_index(long long e, int L, int S, int lines,
-                                                 bool line_major) {
-  if (lines <= 0 || S == 1) return e;
-  const long long slab = static_cast<long long>(L) * S;
-  const long long outer = e / slab;
-  const long long rem = e - outer * slab;
-  const long long j = rem / S;
-  const long long col = rem - j * S;
-  const long long tile = outer * (S / lines) + col / lines;
-  if (line_major) {
-    const int line = static_cast<int>(col % lines);
-    return (tile * lines + line) * L + ((j + amp_line_rotation(L, line)) & (L - 1));
+// otherwise. The modulus pass runs along the slowest axis, so a column is the
+// position within a slab of S = n / L elements.
+struct AmpTiles {
+  int L, S;
+  int lines;  // 0: FFT order
+  bool line_major;
+  __device__ __forceinline__ long long operator()(long long e) const {
+    if (lines <= 0 || S == 1) return e;
+    const int j = static_cast<int>(e / S);
+    const int col = static_cast<int>(e - static_cast<long long>(j) * S);
+    const int line = col % lines;
+    if (line_major) {
+      return static_cast<long long>(col) * L + ((j + amp_line_rotation(L, line)) & (L - 1));
+    }
+    return (static_cast<long long>(col / lines) * L + j) * lines + line;
   }
-  return (tile * L + j) * lines + col % lines;
-}
+};
 
 template <class T>
 __device__ __forceinline__ T from_float(float v);
@@ -112,61 +116,73 @@ __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) {
   return __float2bfloat16_rn(v);
 }
 
+// Blocks of the preparation of one problem, at most: the shares of its energy
+// are added in an order that the shape alone decides.
+constexpr int kPrepareBlocks = 296;
+
+// Sum of the block's values, in thread order of the block; valid in thread 0.
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double partial[kRollThreads / 32];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((tid & 31) == 0) partial[tid >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (tid == 0) {
+    for (int w = 0; w < kRollThreads / 32; ++w) t += partial[w];
+  }
+  return t;
+}
+
+// Everything a solver takes from one centre-origin problem, in one pass over
+// it: the FFT-order amplitude (amp_fft, where it is wanted), the signed
+// amplitude in its storage and tiling, the 0/1 support of `copies` starts and
+// the shares of the usable energy. The seven passes before (three rolls, the
+// sign, the 0/1 step, one block summing the energy alone and a copy per
+// doubling of the supports) took 480 us of a 128^3 problem's reset.
 template <class T>
-__global__ void signed_kernel(const float* amp, const std::uint8_t* mask, long long n, int L, int S,
-                              int lines, bool line_major, T* out) {
-  QPB_LOOP(e, n) {
-    out[tiled_index(e, L, S, lines, line_major)] = from_float<T>(mask[e] ? -1.0f : amp[e]);
-  }
+__global__ void __launch_bounds__(kRollThreads)
+    prepare_problem_kernel(const float* amp, const std::uint8_t* mask, const std::uint8_t* support,
+                           Dims3 d, RollOffsets o, AmpTiles tiles, const float* peak,
+                           float* amp_fft, T* signed_out, std::uint8_t* support_out, int copies,
+                           double* shares) {
+  const long long n = d.n();
+  float unit = 1.0f;
+  if (peak && *peak > 0.0f) unit = *peak;
+  double energy = 0.0;
+  for_rolled(d, o, [&](long long i, long long src, int, int) {
+    float a = amp[src];
+    if (peak) a = a / unit;
+    const bool usable = !(mask && mask[src]);
+    if (amp_fft) amp_fft[i] = a;
+    signed_out[tiles(i)] = from_float<T>(usable ? a : -1.0f);
+    const std::uint8_t inside = support[src] != 0;
+    for (int c = 0; c < copies; ++c) support_out[c * n + i] = inside;
+    if (usable) energy += static_cast<double>(a) * a;
+  });
+  energy = block_sum(energy);
+  if (threadIdx.x == 0 && threadIdx.y == 0) shares[blockIdx.x] = energy;
 }
 
-__global__ void nonzero_kernel(std::uint8_t* v, long long n) {
-  QPB_LOOP(i, n) v[i] = v[i] != 0;
-}
-
-// Usable energy, one block of kEnergyThreads: every element's share is added
-// in the same order on every call.
-constexpr int kEnergyThreads = 1024;
-
-__global__ void __launch_bounds__(kEnergyThreads)
-    energy_kernel(const float* amp, const std::uint8_t* mask, long long n, double* out) {
-  __shared__ double partial[kEnergyThreads / 32];
+// energies[q] = the sum of problem q's `count` shares, always in one order.
+__global__ void energy_kernel(const double* shares, int count, double* energies) {
+  shares += static_cast<long long>(blockIdx.x) * kPrepareBlocks;
   double e = 0.0;
-  for (long long i = threadIdx.x; i < n; i += kEnergyThreads) {
-    if (!mask[i]) e += static_cast<double>(amp[i]) * amp[i];
-  }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = e;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kEnergyThreads / 32; ++w) t += partial[w];
-    *out = t;
-  }
+  for (int i = threadIdx.x; i < count; i += 32) e += shares[i];
+  for (int off = 16; off > 0; off >>= 1) e += __shfl_xor_sync(0xffffffffu, e, off);
+  if (threadIdx.x == 0) energies[blockIdx.x] = e;
 }
 
-// The amplitude's peak (one block; max of non-negative floats by their bits),
-// then amp /= peak, for fp16 storage of the wave: with the peak amplitude at 1
-// the stored transforms stay within fp16 range (the reference's
-// src/cuda/cuda_solver.cu:74-86). A zero amplitude keeps scale 1.
-__global__ void __launch_bounds__(kEnergyThreads)
-    peak_kernel(const float* amp, long long n, float* peak) {
-  __shared__ float partial[kEnergyThreads / 32];
+// The amplitude's peak into `peak` (zeroed before; floats >= 0 order like
+// their bits), which the preparation divides the amplitude by for fp16 storage
+// of the wave: with the peak amplitude at 1 the stored transforms stay within
+// fp16 range (the reference's src/cuda/cuda_solver.cu:74-86). A zero amplitude
+// keeps scale 1.
+__global__ void peak_kernel(const float* amp, long long n, float* peak) {
   float m = 0.0f;
-  for (long long i = threadIdx.x; i < n; i += kEnergyThreads) m = fmaxf(m, amp[i]);
+  QPB_LOOP(i, n) m = fmaxf(m, amp[i]);
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < kEnergyThreads / 32; ++w) t = fmaxf(t, partial[w]);
-    *peak = t > 0.0f ? t : 1.0f;
-  }
-}
-
-__global__ void normalise_kernel(float* amp, long long n, const float* peak) {
-  const float p = *peak;
-  QPB_LOOP(i, n) amp[i] = amp[i] / p;
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(peak), __float_as_int(m));
 }
 
 constexpr std::size_t align256(std::size_t bytes) { return (bytes + 255) / 256 * 256; }
@@ -291,48 +307,53 @@ void autocorrelation_support_host(const float* intensity, int ndim, const long l
   check_waits(operator_plans(), s);
 }
 
-std::size_t prepare_scratch_bytes(long long n) { return align256(static_cast<std::size_t>(n)); }
+std::size_t prepare_share_count() { return kPrepareBlocks; }
 
 void prepare_problem_device(const ProblemView& q, Dims3 d, AmpStorage storage, int L, int S,
                             int lines, bool line_major, float* amp_fft, void* signed_out,
-                            std::uint8_t* support_fft, void* scratch, double* energy,
-                            float* peak, cudaStream_t stream) {
-  const long long n = d.n();
-  std::uint8_t* mask_fft = static_cast<std::uint8_t*>(scratch);
-  roll<float>(q.amplitude, amp_fft, d, 1, true, stream);
+                            std::uint8_t* support_fft, int copies, double* shares, float* peak,
+                            cudaStream_t stream) {
   if (peak) {
-    peak_kernel<<<1, kEnergyThreads, 0, stream>>>(amp_fft, n, peak);
+    QPB_CHECK(cudaMemsetAsync(peak, 0, sizeof(float), stream));
+    peak_kernel<<<blocks_for(d.n()), kThreads, 0, stream>>>(q.amplitude, d.n(), peak);
     QPB_CHECK(cudaGetLastError());
-    normalise_kernel<<<blocks_for(n), kThreads, 0, stream>>>(amp_fft, n, peak);
-    QPB_CHECK(cudaGetLastError());
-    count_launches(2);
+    count_launches(1);
   }
-  if (q.mask) {
-    roll<std::uint8_t>(q.mask, mask_fft, d, 1, true, stream);
-  } else {
-    QPB_CHECK(cudaMemsetAsync(mask_fft, 0, static_cast<std::size_t>(n), stream));
-  }
-  roll<std::uint8_t>(q.support, support_fft, d, 1, true, stream);
-  nonzero_kernel<<<blocks_for(n), kThreads, 0, stream>>>(support_fft, n);
-  QPB_CHECK(cudaGetLastError());
+  auto launch = [&](auto* out) {
+    using T = std::remove_pointer_t<decltype(out)>;
+    prepare_problem_kernel<T><<<roll_blocks(d, kPrepareBlocks), roll_block(d), 0, stream>>>(
+        q.amplitude, q.mask, q.support, d, roll_offsets(d, true), AmpTiles{L, S, lines, line_major},
+        peak, amp_fft, out, support_fft, copies, shares);
+  };
   switch (storage) {
     case AmpStorage::kF32:
-      signed_kernel<float><<<blocks_for(n), kThreads, 0, stream>>>(
-          amp_fft, mask_fft, n, L, S, lines, line_major, static_cast<float*>(signed_out));
+      launch(static_cast<float*>(signed_out));
       break;
     case AmpStorage::kF16:
-      signed_kernel<__half><<<blocks_for(n), kThreads, 0, stream>>>(
-          amp_fft, mask_fft, n, L, S, lines, line_major, static_cast<__half*>(signed_out));
+      launch(static_cast<__half*>(signed_out));
       break;
     case AmpStorage::kBF16:
-      signed_kernel<__nv_bfloat16><<<blocks_for(n), kThreads, 0, stream>>>(
-          amp_fft, mask_fft, n, L, S, lines, line_major, static_cast<__nv_bfloat16*>(signed_out));
+      launch(static_cast<__nv_bfloat16*>(signed_out));
       break;
   }
   QPB_CHECK(cudaGetLastError());
-  energy_kernel<<<1, kEnergyThreads, 0, stream>>>(amp_fft, mask_fft, n, energy);
+  count_launches(1);
+}
+
+void sum_energies(const double* shares, Dims3 d, int problems, double* energies,
+                  cudaStream_t stream) {
+  energy_kernel<<<problems, 32, 0, stream>>>(
+      shares, static_cast<int>(roll_blocks(d, kPrepareBlocks)), energies);
   QPB_CHECK(cudaGetLastError());
-  count_launches(3);
+  count_launches(1);
+}
+
+void configure_device_setup() {
+  prefer_shared_memory(prepare_problem_kernel<float>);
+  prefer_shared_memory(prepare_problem_kernel<__half>);
+  prefer_shared_memory(prepare_problem_kernel<__nv_bfloat16>);
+  prefer_shared_memory(energy_kernel);
+  prefer_shared_memory(peak_kernel);
 }
 
 }  // namespace qpb

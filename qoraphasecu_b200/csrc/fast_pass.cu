@@ -12,8 +12,6 @@
 
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
-#include <set>
 #include <stdexcept>
 
 #include "bulk_copy.cuh"
@@ -572,6 +570,7 @@ int fast_lines(int L, bool rows) {
 template <int L, bool ROWS, Mode M, class AmpT, class WT = float2, class XT = float2>
 void allow_smem_one() {
   constexpr int bytes = Staging<L, ROWS, M, AmpT, WT, XT>::kBytes;
+  prefer_shared_memory(fast_pass_kernel<L, ROWS, M, AmpT, WT, XT>);
   if constexpr (bytes > 48 * 1024) {
     QPB_CHECK(cudaFuncSetAttribute(fast_pass_kernel<L, ROWS, M, AmpT, WT, XT>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -614,20 +613,17 @@ void allow_smem_length() {
 
 }  // namespace
 
-void configure_fast_passes() {
-  static std::mutex mutex;
-  static std::set<int> done;
-  int device = 0;
-  QPB_CHECK(cudaGetDevice(&device));
-  std::lock_guard<std::mutex> lock(mutex);
-  if (!done.insert(device).second) return;
-  allow_smem_length<16>();
-  allow_smem_length<32>();
-  allow_smem_length<64>();
-  allow_smem_length<128>();
-  allow_smem_length<256>();
-  allow_smem_length<512>();
-  allow_smem_length<1024>();
+void configure_fast_pass(int L) {
+  switch (L) {
+    case 16: return allow_smem_length<16>();
+    case 32: return allow_smem_length<32>();
+    case 64: return allow_smem_length<64>();
+    case 128: return allow_smem_length<128>();
+    case 256: return allow_smem_length<256>();
+    case 512: return allow_smem_length<512>();
+    case 1024: return allow_smem_length<1024>();
+    default: return;
+  }
 }
 
 bool fast_passes_enabled() {

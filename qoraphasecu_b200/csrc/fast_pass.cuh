@@ -23,8 +23,8 @@ bool fast_passes_enabled();
 // Lines per CTA of the register-resident kernel for this pass (0: not used).
 int fast_pass_lines(const PassParams& p);
 
-// Raises the dynamic shared-memory limit of the kernels that need more than
-// 48 KiB; once per device, outside stream capture.
-void configure_fast_passes();
+// Sets the shared-memory attributes of the kernels for lines of L points on
+// the current device (configure_line_passes).
+void configure_fast_pass(int L);
 
 }  // namespace qpb

@@ -18,9 +18,13 @@
 #include <mutex>
 #include <set>
 #include <stdexcept>
+#include <utility>
 
+#include "aux_kernels.cuh"
 #include "butterfly.cuh"
 #include "column_pass.cuh"
+#include "dependent_launch.cuh"
+#include "device_setup.cuh"
 #include "fast_pass.cuh"
 #include "line_pass.cuh"
 #include "mixed_pass.cuh"
@@ -304,6 +308,7 @@ constexpr int kMaxPassSmem = 2 * 16 * 512 * static_cast<int>(sizeof(float2));
 template <class Kernel>
 void allow_smem(Kernel kernel) {
   QPB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxPassSmem));
+  prefer_shared_memory(kernel);
 }
 
 template <Mode M>
@@ -337,14 +342,20 @@ void launch_mode(const PassParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-void configure_line_passes() {
-  // Once per device, outside any stream capture.
+namespace {
+
+// The first call of `f` for `key` on the current device.
+template <class F>
+void once_per_device(int key, F&& f) {
   static std::mutex mutex;
-  static std::set<int> done;
+  static std::set<std::pair<int, int>> done;
   int device = 0;
   QPB_CHECK(cudaGetDevice(&device));
   std::lock_guard<std::mutex> lock(mutex);
-  if (!done.insert(device).second) return;
+  if (done.insert({device, key}).second) f();
+}
+
+void configure_generic() {
   allow_smem(line_pass_kernel<Mode::kFwd, float>);
   allow_smem(line_pass_kernel<Mode::kFwdFromX, float>);
   allow_smem(line_pass_kernel<Mode::kInv, float>);
@@ -357,9 +368,31 @@ void configure_line_passes() {
   allow_smem(line_pass_kernel<Mode::kGrad, float>);
   allow_smem(line_pass_kernel<Mode::kGrad, __half>);
   allow_smem(line_pass_kernel<Mode::kGrad, __nv_bfloat16>);
-  configure_fast_passes();
-  configure_column_passes();
-  configure_mixed_passes();
+}
+
+}  // namespace
+
+void configure_line_passes(const PassParams& p) {
+  once_per_device(-2, [] {
+    configure_aux_kernels();
+    configure_device_setup();
+  });
+  // Setting attributes loads a kernel, so each length sets only those its
+  // lines can run (keys: the length, with an offset per kind of pass; 0 to
+  // -2 for the kernels of any length).
+  if (fast_passes_enabled() && fast_pass_supports(p)) {
+    once_per_device(p.L, [&] {
+      configure_fast_pass(p.L);
+      configure_column_pass(p.L);
+    });
+  } else if (fast_passes_enabled() && mixed_pass_supports(p)) {
+    once_per_device(0, [] { configure_mixed_passes(); });
+    once_per_device(p.L + kMaxLine, [&] { configure_two_stage(p.L); });
+    once_per_device(p.L + 2 * kMaxLine, [&] { configure_column_pass(p.L); });
+  } else {
+    once_per_device(-1, [] { configure_generic(); });
+    once_per_device(p.L + 2 * kMaxLine, [&] { configure_column_pass(p.L); });
+  }
 }
 
 int choose_lpc(int L, int S, int lines_per_start) {

@@ -1,8 +1,5 @@
 // Dispatch of the mixed-radix line passes (mixed_pass_kernel.cuh).
 
-#include <mutex>
-#include <set>
-
 #include "mixed_pass.cuh"
 
 namespace qpb {
@@ -34,12 +31,6 @@ void launch_mixed_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
 }
 
 void configure_mixed_passes() {
-  static std::mutex mutex;
-  static std::set<int> done;
-  int device = 0;
-  QPB_CHECK(cudaGetDevice(&device));
-  std::lock_guard<std::mutex> lock(mutex);
-  if (!done.insert(device).second) return;
   configure_mixed_mode<Mode::kFwd>();
   configure_mixed_mode<Mode::kFwdFromX>();
   configure_mixed_mode<Mode::kInv>();

@@ -12,8 +12,8 @@ bool mixed_pass_supports(const PassParams& p);
 
 void launch_mixed_pass(Mode mode, const PassParams& p, cudaStream_t stream);
 
-// Raises the shared-memory limits of the mixed-radix kernels on the current
-// device; called once per device before the first launch (never during capture).
+// Sets the shared-memory attributes of the mixed-radix kernels on the current
+// device (configure_line_passes).
 void configure_mixed_passes();
 
 // The same for one mode (mixed_pass_project.cu, _gradient, _update, _blur and _plain).

@@ -508,8 +508,7 @@ template <Mode M>
 void configure_mixed_mode() {
   auto allow = [](auto kernel) {
     QPB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    QPB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   cudaSharedmemCarveoutMaxShared));
+    prefer_shared_memory(kernel);
   };
   allow(mixed_pass_kernel<M, true>);
   allow(mixed_pass_kernel<M, false>);

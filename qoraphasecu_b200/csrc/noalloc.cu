@@ -24,6 +24,8 @@
 
 #include "../../include/qpb.h"
 #include "bulk_copy.cuh"
+#include "column_pass.cuh"
+#include "fast_pass.cuh"
 #include "fft_plan.hpp"
 #include "line_pass.cuh"
 #include "reduce.cuh"
@@ -69,7 +71,12 @@ ScratchState& scratch_state() {
   if (!state.base) {
     void* ptr = nullptr;
     QPB_CHECK(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
-    configure_line_passes();
+    // every kernel is loaded here, so that no later call has to
+    configure_line_passes(PassParams{});
+    for (int L = 16; L <= 1024; L *= 2) {
+      configure_fast_pass(L);
+      configure_column_pass(L);
+    }
     state.base = static_cast<unsigned char*>(ptr);
   }
   return state;

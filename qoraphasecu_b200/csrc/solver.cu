@@ -28,7 +28,6 @@
 #include "persistent.cuh"
 #include "resident.cuh"
 #include "solver.hpp"
-#include "two_stage_pass.cuh"
 
 namespace qpb {
 
@@ -222,10 +221,9 @@ int recipe_iterations(const OpDesc* ops, std::size_t count) {
 // ------------------------------------------------------------------ PassRunner
 PassRunner::PassRunner(Dims3 d, int ndim, PlanCache& plans)
     : d_(d), ndim_(ndim), wait_failures_(plans.wait_failures()), wait_tries_(kMaxWaitTries) {
-  configure_line_passes();
   for (int a = 0; a < 3; ++a) {
     plans_[a] = (ndim == 2 && a == 0) ? nullptr : &plans.get(axis_len(d, a));
-    if (plans_[a]) configure_two_stage(axis_len(d, a));
+    if (plans_[a]) configure_line_passes(params(Mode::kFwd, a, 1));
   }
 }
 
@@ -373,18 +371,31 @@ Solver::Solver(const std::vector<ProblemView>& problems, const SolverOptions& op
   }
   const std::size_t total = static_cast<std::size_t>(starts_) * n_;
   const std::size_t elem = options.amp_storage == AmpStorage::kF32 ? 4 : 2;
-  amp_ = DeviceBuffer<unsigned char>(static_cast<std::size_t>(problems_) * n_ * elem);
-  amp_f_ = DeviceBuffer<float>(static_cast<std::size_t>(problems_) * n_);
-  support_ = DeviceBuffer<std::uint8_t>(total);
-  x_ = DeviceBuffer<float2>(total);
-  if (iter_half_) xh_ = DeviceBuffer<std::uint32_t>(total);
-  if (fp16_wave_variant()) peaks_ = DeviceBuffer<float>(static_cast<std::size_t>(problems_));
-  w_ = DeviceBuffer<float2>(total);
-  saved_ = DeviceBuffer<std::uint8_t>(total);
-  level_ = DeviceBuffer<LevelAcc>(static_cast<std::size_t>(starts_));
-  moments_ = DeviceBuffer<unsigned long long>(2 * static_cast<std::size_t>(starts_));
-  ctrl_ = DeviceBuffer<Ctrl>(1);
-  counters_ = DeviceBuffer<int>(static_cast<std::size_t>(groups_));
+  const std::size_t amps = static_cast<std::size_t>(problems_) * n_;
+  const auto starts = static_cast<std::size_t>(starts_);
+  // Lays the buffers out from `base`; returns the bytes they take.
+  auto lay_out = [&](unsigned char* base) {
+    std::size_t at = 0;
+    auto take = [&]<class T>(DeviceBuffer<T>& buffer, std::size_t count) {
+      if (base) buffer = DeviceBuffer<T>(reinterpret_cast<T*>(base + at), count);
+      at += (count * sizeof(T) + 255) / 256 * 256;
+    };
+    take(amp_, amps * elem);
+    take(amp_f_, amps);
+    take(support_, total);
+    take(x_, total);
+    if (iter_half_) take(xh_, total);
+    if (fp16_wave_variant()) take(peaks_, static_cast<std::size_t>(problems_));
+    take(w_, total);
+    take(saved_, total);
+    take(level_, starts);
+    take(moments_, 2 * starts);
+    take(ctrl_, 1);
+    take(counters_, static_cast<std::size_t>(groups_));
+    return at;
+  };
+  arena_ = DeviceBuffer<unsigned char>(lay_out(nullptr));
+  lay_out(arena_.get());
   load(problems, options.seed, options.start);
 }
 
@@ -424,26 +435,26 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
   for (const ProblemView& q : problems) {
     if (q.on_device != on_device) throw InvalidArgument("problems mix host and device arrays");
   }
-  // prep_: the problems' energies, then per problem its set-up scratch and,
-  // for host arrays, the staged amplitude, mask and support
+  // prep_: the problems' energies and shares of them, then per problem the
+  // staged amplitude, mask and support of host arrays
   const auto n = static_cast<std::size_t>(n_);
   auto round256 = [](std::size_t b) { return (b + 255) / 256 * 256; };
-  const std::size_t head = round256(static_cast<std::size_t>(problems_) * sizeof(double));
-  const std::size_t scratch = prepare_scratch_bytes(n_);
+  const auto count = static_cast<std::size_t>(problems_);
+  const std::size_t shares = prepare_share_count();
+  const std::size_t head = round256(count * (1 + shares) * sizeof(double));
   const std::size_t amp_bytes = round256(n * sizeof(float));
   const std::size_t staged = on_device ? 0 : amp_bytes + 2 * round256(n);
-  const std::size_t per_problem = scratch + staged;
-  const std::size_t bytes = head + static_cast<std::size_t>(problems_) * per_problem;
+  const std::size_t bytes = head + count * staged;
   if (prep_.size() < bytes) {
     prep_ = DeviceBuffer<unsigned char>();
     prep_ = DeviceBuffer<unsigned char>(bytes);
   }
   auto* energies = reinterpret_cast<double*>(prep_.get());
+  double* all_shares = energies + count;
   for (int q = 0; q < problems_; ++q) {
     ProblemView v = problems[q];
-    unsigned char* region = prep_.get() + head + static_cast<std::size_t>(q) * per_problem;
     if (!on_device) {
-      unsigned char* stage = region + scratch;
+      unsigned char* stage = prep_.get() + head + static_cast<std::size_t>(q) * staged;
       auto* amp = reinterpret_cast<float*>(stage);
       std::uint8_t* mask = stage + amp_bytes;
       std::uint8_t* sup = mask + round256(n);
@@ -458,38 +469,28 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
       v.support = sup;
       v.on_device = true;
     }
-    prepare_problem_device(v, d_, options_.amp_storage, mod.L, mod.S, lines,
-                           amp_tiled_ == kAmpTiledLines,
-                           amp_f_.get() + static_cast<std::size_t>(q) * n_,
-                           amp_.get() + static_cast<std::size_t>(q) * n_ * elem,
-                           support_.get() + static_cast<std::size_t>(q) * spp_ * n_, region,
-                           energies + q, fp16_wave_variant() ? peaks_.get() + q : nullptr,
-                           stream_);
+    prepare_problem_device(
+        v, d_, options_.amp_storage, mod.L, mod.S, lines, amp_tiled_ == kAmpTiledLines,
+        // the FFT-order amplitude is what random starts are drawn on
+        start ? nullptr : amp_f_.get() + static_cast<std::size_t>(q) * n_,
+        amp_.get() + static_cast<std::size_t>(q) * n_ * elem,
+        support_.get() + static_cast<std::size_t>(q) * spp_ * n_, spp_,
+        all_shares + static_cast<std::size_t>(q) * shares,
+        fp16_wave_variant() ? peaks_.get() + q : nullptr, stream_);
   }
-  energies_.assign(static_cast<std::size_t>(problems_), 0.0);
-  QPB_CHECK(cudaMemcpyAsync(energies_.data(), energies, energies_.size() * sizeof(double),
+  sum_energies(all_shares, d_, problems_, energies, stream_);
+  // read back below, by the synchronisation that ends the call
+  host_.reserve(count * (sizeof(double) + sizeof(float)));
+  auto* host_energies = host_.as<double>();
+  auto* host_peaks = reinterpret_cast<float*>(host_energies + count);
+  QPB_CHECK(cudaMemcpyAsync(host_energies, energies, count * sizeof(double),
                             cudaMemcpyDeviceToHost, stream_));
-  amp_scale_.assign(static_cast<std::size_t>(problems_), 1.0f);
   if (fp16_wave_variant()) {
-    QPB_CHECK(cudaMemcpyAsync(amp_scale_.data(), peaks_.get(), amp_scale_.size() * sizeof(float),
+    QPB_CHECK(cudaMemcpyAsync(host_peaks, peaks_.get(), count * sizeof(float),
                               cudaMemcpyDeviceToHost, stream_));
   }
-  QPB_CHECK(cudaMemsetAsync(x_.get(), 0, total * sizeof(float2), stream_));
-  QPB_CHECK(cudaMemsetAsync(counters_.get(), 0, groups_ * sizeof(int), stream_));
-  const Ctrl ctrl{nullptr, 0, 0.0f, 0.0f, counters_.get()};
-  set_ctrl(ctrl_.get(), ctrl, stream_);
-  for (int q = 0; q < problems_; ++q) {
-    std::uint8_t* first = support_.get() + static_cast<std::size_t>(q) * spp_ * n_;
-    // the first start's support to the others, doubling the copied block
-    for (int have = 1; have < spp_;) {
-      const int take = std::min(have, spp_ - have);
-      QPB_CHECK(cudaMemcpyAsync(first + static_cast<std::size_t>(have) * n_, first,
-                                static_cast<std::size_t>(take) * n_, cudaMemcpyDeviceToDevice,
-                                stream_));
-      have += take;
-    }
-  }
-  stream_.sync();
+  qpb::begin_run(ctrl_.get(), Ctrl{nullptr, 0, 0.0f, 0.0f, counters_.get()}, groups_, nullptr, 0,
+                 stream_);
   errors_.assign(static_cast<std::size_t>(starts_), {});
   iteration_ = 0;
   run_iterations_ = 0;
@@ -506,17 +507,18 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
     // Given starts, centre-origin: to FFT order, cut to the support
     // (cpu_solver.cpp:37-41), brought into the scale of an fp16 variant's
     // amplitude (divided by its peak, as test_cuda.cpp:192-205 requires).
-    QPB_CHECK(cudaMemcpyAsync(w_.get(), start, total * sizeof(float2), cudaMemcpyDefault,
-                              stream_));
-    roll<float2>(w_.get(), x_.get(), d_, starts_, true, stream_);
-    support_project(x_.get(), support_.get(), n_, starts_, stream_);
-    if (fp16_wave_variant()) {
-      const std::size_t block = static_cast<std::size_t>(spp_) * n_;
-      for (int q = 0; q < problems_; ++q) {
-        scale_complex(x_.get() + q * block, static_cast<long long>(block),
-                      1.0f / amp_scale_[static_cast<std::size_t>(q)], stream_);
-      }
+    // Aligned starts in this device's memory are read where they are.
+    const float2* from = start;
+    cudaPointerAttributes where{};
+    QPB_CHECK(cudaPointerGetAttributes(&where, start));
+    if (where.type != cudaMemoryTypeDevice || where.device != select_.device ||
+        reinterpret_cast<std::uintptr_t>(start) % alignof(float2) != 0) {
+      QPB_CHECK(cudaMemcpyAsync(w_.get(), start, total * sizeof(float2), cudaMemcpyDefault,
+                                stream_));
+      from = w_.get();
     }
+    roll_cut(from, support_.get(), x_.get(), d_, starts_,
+             fp16_wave_variant() ? peaks_.get() : nullptr, spp_, stream_);
     wave_valid_ = false;
   } else {
     // Random phases on the measured amplitude, inverse transform, cut to the
@@ -532,6 +534,8 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
       p.lines = runner_.params(mode, axis3, count).lines;
       return p;
     };
+    // the update reads the old iterate outside the support
+    QPB_CHECK(cudaMemsetAsync(x_.get(), 0, total * sizeof(float2), stream_));
     for (int g = 0; g < chunks; ++g) {
       random_wave(w(g), amp_f_.get(), amp_stride_, spp_, n_, count, seed,
                   static_cast<std::uint64_t>(g) * batch_, stream_);
@@ -554,6 +558,13 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
   if (wave_half_) wave_valid_ = false;  // the complex64 wave of the starts is not the fp16 one
   if (!wave_valid_) establish_wave();
   stream_.sync();
+  energies_.assign(host_energies, host_energies + problems_);
+  amp_scale_.assign(static_cast<std::size_t>(problems_), 1.0f);
+  if (fp16_wave_variant()) {
+    for (int q = 0; q < problems_; ++q) {
+      if (host_peaks[q] > 0.0f) amp_scale_[q] = host_peaks[q];
+    }
+  }
 }
 
 Solver::~Solver() {
@@ -648,11 +659,8 @@ void Solver::begin_run(const OpDesc* ops, std::size_t count) {
   trace("run: %d iterations, errs %zu -> %zu", iters, errs_.size(), needed);
   if (errs_.size() < needed) errs_ = DeviceBuffer<double>(needed);
   capacity_ = iters;
-  const Ctrl ctrl{errs_.get(), capacity_, 0.0f, 0.0f, counters_.get()};
-  set_ctrl(ctrl_.get(), ctrl, stream_);
-  QPB_CHECK(cudaMemsetAsync(errs_.get(), 0, needed * sizeof(double), stream_));
-  QPB_CHECK(cudaMemsetAsync(counters_.get(), 0, groups_ * sizeof(int), stream_));
-  stream_.sync();
+  qpb::begin_run(ctrl_.get(), Ctrl{errs_.get(), capacity_, 0.0f, 0.0f, counters_.get()}, groups_,
+                 errs_.get(), static_cast<long long>(needed), stream_);
   run_iterations_ = 0;
 }
 
@@ -674,7 +682,6 @@ void Solver::apply(const OpDesc& o) {
 
 void Solver::end_run() {
   collect_errors(run_iterations_);
-  check_waits(plans_, stream_);
 }
 
 void Solver::require_fp16_passes() const {
@@ -1020,18 +1027,25 @@ float Solver::to_error(double num, int start) const {
 
 void Solver::collect_errors(int iterations) {
   trace("collect_errors iterations=%d starts=%d", iterations, starts_);
-  host_errs_.resize(static_cast<std::size_t>(std::max(iterations, 1)) * starts_);
+  // the errors and the passes' failure count, read back by one synchronisation
+  const std::size_t count = static_cast<std::size_t>(iterations) * starts_;
+  host_.reserve((count + 1) * sizeof(double));
+  auto* num = host_.as<double>();
+  auto* failures = reinterpret_cast<int*>(num + count);
   if (iterations > 0) {
-    QPB_CHECK(cudaMemcpyAsync(host_errs_.data(), errs_.get(),
-                              static_cast<std::size_t>(iterations) * starts_ * sizeof(double),
-                              cudaMemcpyDeviceToHost, stream_));
+    QPB_CHECK(cudaMemcpyAsync(num, errs_.get(), count * sizeof(double), cudaMemcpyDeviceToHost,
+                              stream_));
   }
+  QPB_CHECK(cudaMemcpyAsync(failures, plans_.wait_failures(), sizeof(int), cudaMemcpyDeviceToHost,
+                            stream_));
   stream_.sync();
+  const bool failed = *failures != 0;
   for (int t = 0; t < iterations; ++t) {
     for (int s = 0; s < starts_; ++s) {
-      errors_[s].push_back(to_error(host_errs_[static_cast<std::size_t>(t) * starts_ + s], s));
+      errors_[s].push_back(to_error(num[static_cast<std::size_t>(t) * starts_ + s], s));
     }
   }
+  if (failed) check_waits(plans_, stream_);  // clears the count and throws
 }
 
 std::vector<float> Solver::latest_errors() {
@@ -1064,9 +1078,16 @@ void Solver::iterate_f32(float2* out) {
   }
 }
 
-void Solver::results_device(float2* objects, std::uint8_t* supports, float* errors) {
+void Solver::centred(float2* objects, std::uint8_t* supports) {
+  if (objects && supports && !fp16_wave_variant()) {
+    return roll_results(x_.get(), support_.get(), objects, supports, d_, starts_, stream_);
+  }
   if (objects) iterate_f32(objects);
   if (supports) roll<std::uint8_t>(support_.get(), supports, d_, starts_, false, stream_);
+}
+
+void Solver::results_device(float2* objects, std::uint8_t* supports, float* errors) {
+  centred(objects, supports);
   stream_.sync();
   if (errors) {
     const std::size_t count = error_count();
@@ -1095,8 +1116,8 @@ void Solver::results_per_problem(float2* const* objects, std::uint8_t* const* su
   // centre-origin copies on the device, then one transfer per problem
   // straight into the caller's memory
   const std::size_t block = static_cast<std::size_t>(spp_) * n_;
+  centred(objects ? w_.get() : nullptr, supports ? saved_.get() : nullptr);
   if (objects) {
-    iterate_f32(w_.get());
     wave_valid_ = false;
     for (int q = 0; q < problems_; ++q) {
       if (!objects[q]) continue;
@@ -1105,7 +1126,6 @@ void Solver::results_per_problem(float2* const* objects, std::uint8_t* const* su
     }
   }
   if (supports) {
-    roll<std::uint8_t>(support_.get(), saved_.get(), d_, starts_, false, stream_);
     for (int q = 0; q < problems_; ++q) {
       if (!supports[q]) continue;
       QPB_CHECK(cudaMemcpyAsync(supports[q], saved_.get() + q * block, block,

@@ -21,7 +21,8 @@
 
 namespace qpb {
 
-// Owning device allocation.
+// Device memory: an allocation of its own, or a part of another one (which has
+// to outlive it).
 template <class T>
 class DeviceBuffer {
  public:
@@ -38,19 +39,21 @@ class DeviceBuffer {
                                " bytes: " + cudaGetErrorString(status));
     }
   }
+  DeviceBuffer(T* part, std::size_t count) : ptr_(part), count_(count), owned_(false) {}
   DeviceBuffer(const DeviceBuffer&) = delete;
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-  DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), count_(o.count_) {
+  DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), count_(o.count_), owned_(o.owned_) {
     o.ptr_ = nullptr;
     o.count_ = 0;
   }
   DeviceBuffer& operator=(DeviceBuffer&& o) noexcept {
     std::swap(ptr_, o.ptr_);
     std::swap(count_, o.count_);
+    std::swap(owned_, o.owned_);
     return *this;
   }
   ~DeviceBuffer() {
-    if (ptr_) cudaFree(ptr_);
+    if (ptr_ && owned_) cudaFree(ptr_);
   }
   T* get() const { return ptr_; }
   std::size_t size() const { return count_; }
@@ -58,6 +61,36 @@ class DeviceBuffer {
  private:
   T* ptr_ = nullptr;
   std::size_t count_ = 0;
+  bool owned_ = true;
+};
+
+// Page-locked host memory that device copies land in, grown on demand (what it
+// held is lost then).
+class HostBuffer {
+ public:
+  HostBuffer() = default;
+  HostBuffer(const HostBuffer&) = delete;
+  HostBuffer& operator=(const HostBuffer&) = delete;
+  ~HostBuffer() {
+    if (ptr_) cudaFreeHost(ptr_);
+  }
+  void reserve(std::size_t bytes) {
+    if (bytes <= bytes_) return;
+    if (ptr_) cudaFreeHost(ptr_);
+    ptr_ = nullptr;
+    bytes_ = 0;
+    bytes = (bytes + 4095) / 4096 * 4096;
+    QPB_CHECK(cudaMallocHost(&ptr_, bytes));
+    bytes_ = bytes;
+  }
+  template <class T>
+  T* as() const {
+    return static_cast<T*>(ptr_);
+  }
+
+ private:
+  void* ptr_ = nullptr;
+  std::size_t bytes_ = 0;
 };
 
 // A stream the object creates (and destroys), or one the caller lends.
@@ -340,6 +373,9 @@ class Solver {
   // it) into `out` (starts * numel): widened from fp16 and multiplied back by
   // each problem's amplitude peak where the variant stores it so.
   void iterate_f32(float2* out);
+  // The iterate (complex64, unscaled) and the supports, centre-origin, into
+  // device memory; a null array is left out.
+  void centred(float2* objects, std::uint8_t* supports);
   void report();
   float to_error(double num, int start) const;
 
@@ -357,10 +393,13 @@ class Solver {
   Stream stream_;
   PassRunner runner_;
   std::vector<double> energies_;     // usable energy per problem
+  // One allocation for the buffers below up to counters_ (an allocation of
+  // more than a megabyte costs about 0.35 ms, and as much to free).
+  DeviceBuffer<unsigned char> arena_;
   long long amp_stride_ = 0;         // elements between problems' amplitudes in amp_
   DeviceBuffer<unsigned char> amp_;  // signed amplitude in the chosen storage
   DeviceBuffer<float> amp_f_;        // FP32 FFT-order amplitude, for the random starts
-  DeviceBuffer<unsigned char> prep_;  // problem set-up: scratch, and host arrays staged
+  DeviceBuffer<unsigned char> prep_;  // problem set-up: energies, and host arrays staged
   int amp_tiled_ = 0;                // amp_ in the modulus pass's CTA order (kAmpTiled*)
   bool resident_ = false;            // iterations run by the resident kernel
   bool persistent_ = false;          // iterations run by the persistent kernel
@@ -386,7 +425,7 @@ class Solver {
   std::vector<std::unique_ptr<Stream>> branches_;
   std::vector<cudaEvent_t> branch_events_;
   std::vector<std::vector<float>> errors_;
-  std::vector<double> host_errs_;
+  HostBuffer host_;  // what load() and collect_errors() read back
   int iteration_ = 0;
   int run_iterations_ = 0;
   ProgressFn progress_ = nullptr;

@@ -258,10 +258,7 @@ void configure_one() {
   static_assert(bytes <= 226 * 1024);
   QPB_CHECK(cudaFuncSetAttribute(two_stage_kernel<L, M, ROWS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  // one carve-out for all: a change between passes drains the SMs
-  QPB_CHECK(cudaFuncSetAttribute(two_stage_kernel<L, M, ROWS>,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared));
+  prefer_shared_memory(two_stage_kernel<L, M, ROWS>);
 }
 
 constexpr int two_stage_count(int slice) {

@@ -1,9 +1,6 @@
 // Dispatch of the two-stage line passes (two_stage_kernel.cuh).
 
 #include <array>
-#include <mutex>
-#include <set>
-#include <utility>
 
 #include "two_stage_pass.cuh"
 
@@ -60,12 +57,6 @@ void launch_two_stage_pass(Mode mode, const PassParams& p, cudaStream_t stream) 
 }
 
 void configure_two_stage(int L) {
-  static std::mutex mutex;
-  static std::set<std::pair<int, int>> done;
-  int device = 0;
-  QPB_CHECK(cudaGetDevice(&device));
-  std::lock_guard<std::mutex> lock(mutex);
-  if (!done.insert({device, L}).second) return;
   for (const Mode mode : {Mode::kUpd, Mode::kFwdFromX, Mode::kInv, Mode::kMod, Mode::kGrad,
                           Mode::kFwd}) {
     for (const bool rows : {false, true}) {

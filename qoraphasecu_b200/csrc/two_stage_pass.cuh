@@ -30,8 +30,8 @@ bool two_stage_supports(Mode mode, const PassParams& p);
 
 void launch_two_stage_pass(Mode mode, const PassParams& p, cudaStream_t stream);
 
-// Raises the shared-memory limits of the passes of length L on the current
-// device; called before their first launch (never during capture).
+// Sets the shared-memory attributes of the passes of length L on the current
+// device (configure_line_passes).
 void configure_two_stage(int L);
 
 }  // namespace qpb
