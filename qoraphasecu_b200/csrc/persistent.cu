@@ -191,7 +191,8 @@ struct WorkList {
   unsigned* work;
 };
 
-template <int LY, int LX>
+// AmpT: the amplitude's storage (its tile takes the space of a float one).
+template <int LY, int LX, class AmpT>
 __global__ void __launch_bounds__(Persist<LY, LX>::NT, Persist<LY, LX>::MIN_CTAS)
     persistent_kernel(const __grid_constant__ CUtensorMap wmap, const PassParams mod,
                       const PassParams upd, const WorkList wl) {
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(Persist<LY, LX>::NT, Persist<LY, LX>::MIN_CTAS
     bool ok;
     unsigned* done;
     if (rem < modulus_items) {
-      ok = column_tile<LY, Mode::kMod, float, float2, kColumnLines, false>(
+      ok = column_tile<LY, Mode::kMod, AmpT, float2, kColumnLines, false>(
           &wmap, mod, static_cast<long long>(rem), cs, parity_c, row0 + static_cast<int>(i));
       parity_c ^= 1u;
       done = done_c + rem / wl.tiles_c;
@@ -316,8 +317,8 @@ __global__ void __launch_bounds__(Persist<LY, LX>::NT, Persist<LY, LX>::MIN_CTAS
   }
 }
 
-template <int LY, int LX>
-void launch_shape(const PassParams& mod, const PassParams& upd, int starts, int iterations,
+template <int LY, int LX, class AmpT>
+void launch_storage(const PassParams& mod, const PassParams& upd, int starts, int iterations,
                   unsigned* work, cudaStream_t stream) {
   using P = Persist<LY, LX>;
   static_assert(P::ROWS >= 1, "rows per update tile");
@@ -326,8 +327,8 @@ void launch_shape(const PassParams& mod, const PassParams& upd, int starts, int 
   int device = 0, sms = 0, per_sm = 0;
   QPB_CHECK(cudaGetDevice(&device));
   QPB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  QPB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_kernel<LY, LX>,
-                                                          P::NT, P::kBytes));
+  QPB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, persistent_kernel<LY, LX, AmpT>, P::NT, P::kBytes));
   const long long items = static_cast<long long>(starts) * (wl.tiles_c + wl.tiles_r) * iterations;
   const int grid = static_cast<int>(std::min<long long>(static_cast<long long>(sms) * std::max(per_sm, 1),
                                                         items));
@@ -342,16 +343,33 @@ void launch_shape(const PassParams& mod, const PassParams& upd, int starts, int 
   attr.val.cooperative = 1;
   config.attrs = &attr;
   config.numAttrs = 1;
-  QPB_CHECK(cudaLaunchKernelEx(&config, persistent_kernel<LY, LX>, map, mod, upd, wl));
+  QPB_CHECK(cudaLaunchKernelEx(&config, persistent_kernel<LY, LX, AmpT>, map, mod, upd, wl));
   count_launches(1);
+}
+
+template <int LY, int LX>
+void launch_shape(const PassParams& mod, const PassParams& upd, int starts, int iterations,
+                  unsigned* work, cudaStream_t stream) {
+  switch (mod.amp_storage) {
+    case AmpStorage::kF32:
+      return launch_storage<LY, LX, float>(mod, upd, starts, iterations, work, stream);
+    case AmpStorage::kF16:
+      return launch_storage<LY, LX, __half>(mod, upd, starts, iterations, work, stream);
+    case AmpStorage::kBF16:
+      return launch_storage<LY, LX, __nv_bfloat16>(mod, upd, starts, iterations, work, stream);
+  }
 }
 
 template <int LY, int LX>
 void allow_shape() {
   constexpr int bytes = Persist<LY, LX>::kBytes;
   if constexpr (bytes > 48 * 1024) {
-    QPB_CHECK(cudaFuncSetAttribute(persistent_kernel<LY, LX>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    auto allow = [](auto kernel) {
+      QPB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    };
+    allow(persistent_kernel<LY, LX, float>);
+    allow(persistent_kernel<LY, LX, __half>);
+    allow(persistent_kernel<LY, LX, __nv_bfloat16>);
   }
 }
 
@@ -376,9 +394,9 @@ int grid_y(int lx) {
     return sms * per_sm;
   };
   switch (lx) {
-    case 64: return grid(persistent_kernel<LY, 64>, Persist<LY, 64>::NT, Persist<LY, 64>::kBytes);
-    case 128: return grid(persistent_kernel<LY, 128>, Persist<LY, 128>::NT, Persist<LY, 128>::kBytes);
-    case 256: return grid(persistent_kernel<LY, 256>, Persist<LY, 256>::NT, Persist<LY, 256>::kBytes);
+    case 64: return grid(persistent_kernel<LY, 64, float>, Persist<LY, 64>::NT, Persist<LY, 64>::kBytes);
+    case 128: return grid(persistent_kernel<LY, 128, float>, Persist<LY, 128>::NT, Persist<LY, 128>::kBytes);
+    case 256: return grid(persistent_kernel<LY, 256, float>, Persist<LY, 256>::NT, Persist<LY, 256>::kBytes);
     default: return 0;
   }
 }
