@@ -52,15 +52,32 @@ QPB_HD float fftfreq(std::uint32_t k, std::uint32_t n) {
 }
 
 // ---------------------------------------------------------------- complex
-QPB_HD float2 cadd(float2 a, float2 b) { return {a.x + b.x, a.y + b.y}; }
-QPB_HD float2 csub(float2 a, float2 b) { return {a.x - b.x, a.y - b.y}; }
-QPB_HD float2 cscale(float2 a, float s) { return {a.x * s, a.y * s}; }
-QPB_HD float2 cmul(float2 a, float2 b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+// Both components in one packed instruction where they meet the same
+// operation (two FP32 values an instruction on sm_100), each rounded as the
+// scalar operation would be; nothing here is left to the compiler to contract.
+#ifdef __CUDACC__
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// a - b, as the exact product with -1 in an FMA
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  return __ffma2_rn(b, float2{-1.0f, -1.0f}, a);
+}
+__device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, float2{s, s}); }
+// s a + b
+__device__ __forceinline__ float2 cfma(float s, float2 a, float2 b) {
+  return __ffma2_rn(float2{s, s}, a, b);
+}
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  return {fmaf(-a.y, b.y, __fmul_rn(a.x, b.x)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y))};
+}
 // a * conj(b)
-QPB_HD float2 cmulc(float2 a, float2 b) { return {a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y}; }
-// a * (-i) and a * (+i)
-QPB_HD float2 mul_mi(float2 a) { return {a.y, -a.x}; }
-QPB_HD float2 mul_pi(float2 a) { return {-a.y, a.x}; }
+__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
+  return {fmaf(a.y, b.y, __fmul_rn(a.x, b.x)), fmaf(-a.x, b.y, __fmul_rn(a.y, b.x))};
+}
+// The update outside the support, a x + b P.
+__device__ __forceinline__ float2 relaxed(float a, float2 x, float b, float2 projected) {
+  return cfma(a, x, cscale(projected, b));
+}
+#endif
 
 // ---------------------------------------------------------------- errors
 // Status codes of the C ABI (include/qpb.h).

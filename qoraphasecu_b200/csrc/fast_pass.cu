@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
         float2 xn = kHalfStorage<WT> ? cscale(v[m], p.scale) : v[m];
         if (!s_tile[l * St::kSupportPitch + t + T * m]) {
           const float2 xo = load_c(x_tile[j]);
-          xn = {ca * xo.x + cb * xn.x, ca * xo.y + cb * xn.y};
+          xn = relaxed(ca, xo, cb, xn);
         }
         x_tile[j] = store_c<XT>(xn);
         v[m] = xn;
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
         float2 xn = kHalfStorage<WT> ? cscale(v[m], p.scale) : v[m];
         if (!sl[m * step]) {
           const float2 xo = load_c(xl[m * step]);
-          xn = {ca * xo.x + cb * xn.x, ca * xo.y + cb * xn.y};
+          xn = relaxed(ca, xo, cb, xn);
         }
         xl[m * step] = store_c<XT>(xn);
         v[m] = xn;

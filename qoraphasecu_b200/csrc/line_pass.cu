@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads) line_pass_kernel(const PassParams p)
       float2 xn = pv;
       if (!p.support[g]) {
         const float2 xo = p.x[g];
-        xn = {ca * xo.x + cb * pv.x, ca * xo.y + cb * pv.y};
+        xn = relaxed(ca, xo, cb, pv);
       }
       p.x[g] = xn;
       res[l * ldl + j] = xn;

@@ -216,7 +216,7 @@ struct MixedPass {
           const int q = q0 + b;
           if (q < R) {
             if (side.outside >> q & 1u) {
-              v[q] = {ca * xo[b].x + cb * v[q].x, ca * xo[b].y + cb * v[q].y};
+              v[q] = relaxed(ca, xo[b], cb, v[q]);
             }
             x[e + q * step] = v[q];
           }

@@ -159,7 +159,7 @@ __device__ __forceinline__ bool update_tile(const PassParams& p, long long tile,
     float2 xn = v[m];
     if (!s_tile[j]) {
       const float2 xo = x_tile[j];
-      xn = {ca * xo.x + cb * xn.x, ca * xo.y + cb * xn.y};
+      xn = relaxed(ca, xo, cb, xn);
     }
     x_tile[j] = xn;
     v[m] = xn;

@@ -38,7 +38,7 @@ __device__ __forceinline__ float divide(float a, float b) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
   const float e = fmaf(-b, y, 1.0f);
   y = fmaf(e, y, y);
-  const float q = a * y;
+  const float q = __fmul_rn(a, y);
   const float r = fmaf(-b, q, a);
   return fmaf(r, y, q);
 }
@@ -57,9 +57,9 @@ __device__ __forceinline__ float square_root(float x) {
   const float xs = tiny ? x * 0x1p64f : x;
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(xs));
-  const float s = xs * y;
+  const float s = __fmul_rn(xs, y);
   const float r = fmaf(-s, s, xs);
-  const float q = fmaf(r, 0.5f * y, s);
+  const float q = fmaf(r, __fmul_rn(0.5f, y), s);
   return xs > 0.0f ? (tiny ? q * 0x1p-32f : q) : 0.0f;
 }
 
@@ -78,30 +78,29 @@ __device__ __forceinline__ float square_root(float x) {
 template <Mode M>
 __device__ __forceinline__ float2 pointwise_projection(float2 v, float a, float s, float& acc,
                                                        float out_scale) {
-  const float re = v.x * s;
-  const float im = v.y * s;
+  const float2 y = cscale(v, s);
   // The reference's expression (src/cuda/device.cuh:20-27): the square root
   // of the squared magnitude and the quotient by (|y| + eps), each within one
   // ulp of the IEEE operation.
-  const float mag = square_root(re * re + im * im);
+  const float mag = square_root(fmaf(y.y, y.y, __fmul_rn(y.x, y.x)));
   float f;
   if constexpr (M == Mode::kGrad) {
     f = 0.0f;
     if (a >= 0.0f) {
       const float d = mag - a;
-      acc += d * d;
-      f = 2.0f * (1.0f - divide(a, mag + kEps)) * out_scale;
+      acc = fmaf(d, d, acc);
+      f = __fmul_rn(__fmul_rn(2.0f, __fsub_rn(1.0f, divide(a, mag + kEps))), out_scale);
     }
   } else {
     float target = mag;
     if (a >= 0.0f) {
       const float d = mag - a;
-      acc += d * d;
+      acc = fmaf(d, d, acc);
       target = a;
     }
-    f = divide(target, mag + kEps) * out_scale;
+    f = __fmul_rn(divide(target, mag + kEps), out_scale);
   }
-  return {re * f, im * f};
+  return cscale(y, f);
 }
 
 template <Mode M>

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(Resident<N>::NT, 1) resident_kernel(const Resi
       float2 xn = v[m];
       if (!ss[j]) {
         const float2 xo = xs[j];
-        xn = {ca * xo.x + cb * xn.x, ca * xo.y + cb * xn.y};
+        xn = relaxed(ca, xo, cb, xn);
       }
       xs[j] = xn;
       v[m] = xn;

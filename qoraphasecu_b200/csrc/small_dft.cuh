@@ -74,12 +74,11 @@ __device__ __forceinline__ void dft_odd_prime(float2* v) {
       constexpr int i = ii;
       constexpr float c = static_cast<float>(turn_cosine((i + 1) * m, R));
       constexpr float d = static_cast<float>(turn_sine((i + 1) * m, R));
-      r = {fmaf(c, a[i].x, r.x), fmaf(c, a[i].y, r.y)};
-      s = {fmaf(d, b[i].x, s.x), fmaf(d, b[i].y, s.y)};
+      r = cfma(c, a[i], r);
+      s = i == 0 ? cscale(b[i], d) : cfma(d, b[i], s);
     });
-    const float2 q = mul_w4<INV>(s);
-    v[m] = cadd(r, q);
-    v[R - m] = csub(r, q);
+    v[m] = cadd_w4<INV>(r, s);
+    v[R - m] = csub_w4<INV>(r, s);
   });
 }
 
@@ -132,8 +131,8 @@ __device__ __forceinline__ void dft_square(float2* v) {
     unrolled<P - 1>([&](auto k) {
       constexpr int e = (i + 1) * (k + 1);
       constexpr float c = static_cast<float>(turn_cosine(e, R));
-      constexpr float s = static_cast<float>(turn_sine(INV ? e : -e, R));
-      t[i + 1][k + 1] = cmul(t[i + 1][k + 1], float2{c, s});
+      constexpr float s = static_cast<float>(turn_sine(e, R));
+      t[i + 1][k + 1] = cmul_constant<INV>(t[i + 1][k + 1], c, s);
     });
   });
 #pragma unroll

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
 #pragma unroll
       for (int q = 0; q < B; ++q) {
         const float2 xo = side[q * lpc * T + tid];
-        if (!inside[q]) u[q] = {ca * xo.x + cb * u[q].x, ca * xo.y + cb * u[q].y};
+        if (!inside[q]) u[q] = relaxed(ca, xo, cb, u[q]);
         x[q * A * S] = u[q];
       }
     } else {
