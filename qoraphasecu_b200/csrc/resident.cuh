@@ -26,23 +26,30 @@ struct ResidentParams {
   int iterations;                // iterations this launch runs
   float scale;                   // 1/N (= 1/sqrt(n))
   AmpStorage amp_storage;
+  int cluster;                   // CTAs per start (resident_cluster)
 };
 
 // Side lengths with a resident kernel (square 2D problems only): 64, 128, 256.
 bool resident_supports(int ndim, int d1, int d2);
 
-// CTAs per start (the cluster size) for side N.
-int resident_cluster(int side);
+// CTAs per start (the cluster size) for `starts` starts of side N on the
+// current device: the largest size at which every start is resident at once
+// with one CTA per SM, else the smallest. More SMs per start shorten an
+// iteration's serial chain as long as they would be idle otherwise.
+int resident_cluster(int side, int starts);
 
-// Clusters of the side-N kernel that the current device runs at once.
-int resident_max_clusters(int side);
+// Clusters of that size of the side-N kernel that the current device runs at once.
+int resident_max_clusters(int side, int cluster);
 
 // Enqueues `p.iterations` iterations of `starts` starts of an N x N problem, then
 // advances ctrl->counters[group] by that count.
 void launch_resident(const ResidentParams& p, int side, int starts, cudaStream_t stream);
 
-// Raises the shared-memory limits of the resident kernels on the current device
-// (once per device, outside stream capture).
-void configure_resident();
+// The smallest cluster a start of side N fits.
+int resident_smallest_cluster(int side);
+
+// Sets the attributes of side N's kernels on the current device (once per
+// device, outside stream capture; resident_cluster does so too).
+void configure_resident(int side);
 
 }  // namespace qpb

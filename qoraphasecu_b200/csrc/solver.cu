@@ -346,7 +346,7 @@ Solver::Solver(const std::vector<ProblemView>& problems, const SolverOptions& op
   }
   if (resident_ || persistent_) batch_ = starts_;
   groups_ = starts_ / batch_;
-  if (resident_) configure_resident();
+  if (resident_) cluster_ = resident_cluster(d_.d2, starts_);
   if (persistent_) {
     configure_persistent();
     work_ = DeviceBuffer<unsigned>(static_cast<std::size_t>(persistent_work_words(starts_)));
@@ -644,6 +644,7 @@ void Solver::enqueue_chunk(int len, cudaStream_t s) {
   p.iterations = len;
   p.scale = 1.0f / static_cast<float>(d_.d2);
   p.amp_storage = options_.amp_storage;
+  p.cluster = cluster_;
   launch_resident(p, d_.d2, starts_, s);
 }
 
@@ -823,8 +824,11 @@ void Solver::end_chunk(int len) {
 void Solver::iterate(int count, Coefficients c) {
   begin_iterate(c);
   for (int done = 0; done < count;) {
-    const int len = chunk_length(count - done);
-    if (batched()) {
+    // the resident kernel runs a stage in one launch unless someone watches
+    const int len = resident_ && !progress_ ? count - done : chunk_length(count - done);
+    if (resident_) {
+      enqueue_chunk_body(len, stream_);
+    } else if (batched()) {
       // graphs by chunk length and wave storage (the mixed variant switches it)
       const int key = 2 * len + (wave_half_ ? 1 : 0);
       auto it = graphs_.find(key);

@@ -402,6 +402,7 @@ class Solver {
   DeviceBuffer<unsigned char> prep_;  // problem set-up: energies, and host arrays staged
   int amp_tiled_ = 0;                // amp_ in the modulus pass's CTA order (kAmpTiled*)
   bool resident_ = false;            // iterations run by the resident kernel
+  int cluster_ = 0;                  // its CTAs per start
   bool persistent_ = false;          // iterations run by the persistent kernel
   DeviceBuffer<unsigned> work_;      // the persistent kernel's work-list words
   DeviceBuffer<float2> x_;

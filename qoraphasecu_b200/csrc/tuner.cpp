@@ -148,8 +148,10 @@ std::string tuning_report() {
     bool first = true;
     for (const auto& [batch, t] : g_timings[key]) {
       if (batch == 0) {
-        out << (first ? "" : ", ") << "resident (" << resident_max_clusters(d2) << " clusters of "
-            << resident_cluster(d2) << " CTAs at once): " << t * 1e3 << " ms";
+        const int smallest = resident_smallest_cluster(d2);
+        out << (first ? "" : ", ") << "resident (" << resident_max_clusters(d2, smallest)
+            << " clusters of " << smallest << " CTAs at once, " << resident_cluster(d2, starts)
+            << " CTAs a start taken): " << t * 1e3 << " ms";
       } else if (batch == kPersistentCandidate) {
         out << (first ? "" : ", ") << "persistent (" << persistent_grid(d1, d2)
             << " CTAs): " << t * 1e3 << " ms";
