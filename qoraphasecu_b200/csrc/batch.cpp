@@ -128,8 +128,7 @@ void BatchSolver::run(const OpDesc* ops, std::size_t count) {
     for (int done = 0; done < o.n;) {
       const int len = classes_[0].solver->chunk_length(o.n - done);
       if (batched_) {
-        // graphs by chunk length and wave storage (the mixed variant switches it)
-        const int key = 2 * len + (classes_[0].solver->wave_half() ? 1 : 0);
+        const int key = classes_[0].solver->graph_key(len);
         auto it = graphs_.find(key);
         if (it == graphs_.end()) {
           for (Class& c : classes_) c.solver->prepare_branches();

@@ -68,9 +68,11 @@ struct Staging {
   using G = Tiling<L, ROWS>;
   using InT = std::conditional_t<M == Mode::kFwdFromX, XT, WT>;
   static constexpr bool kRowTma =
-      ROWS && (M == Mode::kFwd || M == Mode::kFwdFromX || M == Mode::kInv || M == Mode::kUpd);
+      ROWS && (M == Mode::kFwd || M == Mode::kFwdFromX || M == Mode::kInv || M == Mode::kUpd ||
+               M == Mode::kCut);
   static constexpr bool kAmp = M == Mode::kMod || M == Mode::kGrad;
-  static constexpr bool kUpd = M == Mode::kUpd && ROWS;
+  static constexpr bool kUpd = M == Mode::kUpd && ROWS;    // reads and writes the iterate
+  static constexpr bool kSupport = ROWS && (M == Mode::kUpd || M == Mode::kCut);
   // Rows of 128 points (8 threads a row, a half-warp holding two rows) sit
   // kRowPitch elements apart in the staged wave, iterate and output tiles, one
   // bulk copy per row, and the exchange rows kXPitch = 8 mod 16 values apart,
@@ -101,11 +103,11 @@ struct Staging {
   // more there (11.26 -> 11.57 us for 32 starts of 256^2).
   static constexpr int kSupportPitch = G::LINES > 1 && L <= 128 ? L + 16 : L;
   static constexpr int kSupportBytes = G::LINES * L;  // bytes the copies deliver
-  static constexpr int kSideB = kUpd ? G::LINES * kSupportPitch : 0;
+  static constexpr int kSideB = kSupport ? G::LINES * kSupportPitch : 0;
   static constexpr bool kBarrierUsed = kAmp || kUpd || kRowTma;
   // A row update (two transforms per tile) reads its twiddles from a copy of
   // the stage-major table in shared memory, copied with the wave tile.
-  static constexpr bool kTwStaged = kUpd && Geometry<L>::STAGES > 1 && L <= 256;
+  static constexpr bool kTwStaged = kSupport && Geometry<L>::STAGES > 1 && L <= 256;
   static constexpr int kTwOffset = align16(kExchange + kSideA + kSideB);
   static constexpr int kTwBytes = kTwStaged ? Geometry<L>::TW_COUNT * 8 : 0;
   static constexpr int kBarrier = align16(kTwOffset + kTwBytes);
@@ -195,11 +197,11 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
   // the old iterate and support of a row update, which are needed only after
   // the inverse transform, so their copies overlap it.
   [[maybe_unused]] auto* bar = reinterpret_cast<std::uint64_t*>(sbase + St::kBarrier);
-  [[maybe_unused]] std::uint64_t* side_bar = St::kUpd ? bar + 1 : bar;
+  [[maybe_unused]] std::uint64_t* side_bar = St::kSupport ? bar + 1 : bar;
   if constexpr (St::kBarrierUsed) {
     if (tid == 0) {
       mbar_init(bar, 1);
-      if constexpr (St::kUpd) {
+      if constexpr (St::kSupport) {
         mbar_arrive_expect_tx(bar, St::kTileIn + St::kTwBytes);
         mbar_init(side_bar, 1);
         mbar_arrive_expect_tx(side_bar, St::kSideABytes + St::kSupportBytes);
@@ -226,16 +228,18 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
         }
       }
     }
-    if constexpr (St::kUpd) {
+    if constexpr (St::kSupport) {
       if (tid == 0 && !p.starve) {
-        const XT* xsrc = reinterpret_cast<const XT*>(p.x) + line0 * L;
-        if constexpr (St::kPadRows) {
-          for (int r = 0; r < Ti::LINES; ++r) {
-            bulk_g2s(reinterpret_cast<XT*>(sbase + St::kExchange) + r * St::kRowPitch,
-                     xsrc + r * L, L * static_cast<int>(sizeof(XT)), side_bar);
+        if constexpr (St::kUpd) {
+          const XT* xsrc = reinterpret_cast<const XT*>(p.x) + line0 * L;
+          if constexpr (St::kPadRows) {
+            for (int r = 0; r < Ti::LINES; ++r) {
+              bulk_g2s(reinterpret_cast<XT*>(sbase + St::kExchange) + r * St::kRowPitch,
+                       xsrc + r * L, L * static_cast<int>(sizeof(XT)), side_bar);
+            }
+          } else {
+            bulk_g2s(sbase + St::kExchange, xsrc, St::kSideA, side_bar);
           }
-        } else {
-          bulk_g2s(sbase + St::kExchange, xsrc, St::kSideA, side_bar);
         }
         if constexpr (St::kSupportPitch == L) {
           bulk_g2s(sbase + St::kExchange + St::kSideA, p.support + line0 * L, St::kSupportBytes,
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
     if (!__syncthreads_and(mbar_wait(b, 0, p.wait_tries) ? 1 : 0)) {
       if (tid == 0) {
         mbar_wait(bar, 0, p.wait_tries);
-        if constexpr (St::kUpd) mbar_wait(side_bar, 0, p.wait_tries);
+        if constexpr (St::kSupport) mbar_wait(side_bar, 0, p.wait_tries);
         atomicAdd(p.wait_failures, 1);
       }
       return false;
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
     }
   }
 
-  constexpr bool kStartsInverse = M == Mode::kInv || M == Mode::kUpd;
+  constexpr bool kStartsInverse = M == Mode::kInv || M == Mode::kUpd || M == Mode::kCut;
   // The last exchange's closing barrier is needed only before a second
   // transform with no block barrier in between (the blur's); a modulus pass
   // passes one in its error sum, an update in its store, and the passes of a
@@ -382,6 +386,18 @@ __global__ void __launch_bounds__(Tiling<L, ROWS>::NT, Tiling<L, ROWS>::MIN_CTAS
       __syncthreads();
     }
     if (p.bump_counter && blockIdx.x == 0 && tid == 0) ++p.ctrl->counters[p.group];
+    transform<L, false, kWarpLocal, false, kTwShared>(v, t, tw, row);
+  } else if constexpr (M == Mode::kCut) {
+    static_assert(ROWS, "updates run along rows");
+    if (!staged(side_bar)) return;
+    const std::uint8_t* s_tile = sbase + St::kExchange + St::kSideA;
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      if constexpr (kHalfStorage<WT>) v[m] = cscale(v[m], p.scale);
+      if (!s_tile[l * St::kSupportPitch + t + T * m]) v[m] = cscale(v[m], 0.0f);
+    }
+    if (p.bump_counter && blockIdx.x == 0 && tid == 0) ++p.ctrl->counters[p.group];
+    // (the staged wait's block barrier is past every exchange read)
     transform<L, false, kWarpLocal, false, kTwShared>(v, t, tw, row);
   } else if constexpr (M == Mode::kBlur || M == Mode::kBlurMag) {
     const float inv_l = 1.0f / static_cast<float>(L);
@@ -464,7 +480,8 @@ void launch_one(const PassParams& p, cudaStream_t stream) {
 // either iterate storage.
 template <Mode M>
 inline constexpr bool kHalfWaveMode = M == Mode::kFwd || M == Mode::kFwdFromX ||
-                                      M == Mode::kInv || M == Mode::kMod || M == Mode::kUpd;
+                                      M == Mode::kInv || M == Mode::kMod || M == Mode::kUpd ||
+                                      M == Mode::kCut;
 template <Mode M>
 inline constexpr bool kTouchesX = M == Mode::kFwdFromX || M == Mode::kUpd || M == Mode::kBlurMag;
 
@@ -514,6 +531,9 @@ void launch_mode(Mode mode, const PassParams& p, cudaStream_t stream) {
       return launch_storage<L, ROWS, Mode::kMod>(p, stream);
     case Mode::kUpd:
       return launch_storage<L, ROWS, Mode::kUpd>(p, stream);
+    case Mode::kCut:
+      if constexpr (ROWS) return launch_storage<L, ROWS, Mode::kCut>(p, stream);
+      throw std::logic_error("fast line pass: updates run along rows");
     case Mode::kBlur:
       return launch_storage<L, ROWS, Mode::kBlur>(p, stream);
     case Mode::kBlurMag:
@@ -592,6 +612,10 @@ void allow_smem_modes() {
   allow_smem_one<L, ROWS, Mode::kMod, __half>();
   allow_smem_one<L, ROWS, Mode::kMod, __nv_bfloat16>();
   allow_smem_one<L, ROWS, Mode::kUpd, float>();
+  if constexpr (ROWS) {
+    allow_smem_one<L, ROWS, Mode::kCut, float>();
+    allow_smem_half<L, ROWS, Mode::kCut>();
+  }
   allow_smem_one<L, ROWS, Mode::kBlur, float>();
   allow_smem_one<L, ROWS, Mode::kBlurMag, float>();
   allow_smem_one<L, ROWS, Mode::kGrad, float>();

@@ -440,6 +440,7 @@ void launch_line_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
     case Mode::kMod:
       return launch_mode<Mode::kMod>(p, stream);
     case Mode::kUpd:
+    case Mode::kCut:  // with the control block's coefficients of error reduction, 0 and 0
       return launch_mode<Mode::kUpd>(p, stream);
     case Mode::kBlur:
       return launch_mode<Mode::kBlur>(p, stream);

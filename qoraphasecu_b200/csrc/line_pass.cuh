@@ -23,6 +23,7 @@ enum class Mode : int {
   kInv,      // w <- IFFT(w)
   kMod,      // w <- IFFT(P_M FFT(w)) and the Fourier-error numerator per start
   kUpd,      // P <- IFFT(w); x <- S ? P : a x + b P; w <- FFT(x)
+  kCut,      // w <- FFT(S ? IFFT(w) : 0): an error-reduction update that leaves x as it was
   kBlur,     // w <- IFFT(g FFT(w)), g = exp(k f^2) / L along this axis
   kBlurMag,  // as kBlur on (|x|, 0)
   kGrad,     // w <- IFFT(2 (1 - A / (|y| + eps)) y), y = FFT(w), and sum (|y| - A)^2:

@@ -21,6 +21,8 @@ void launch_mixed_pass(Mode mode, const PassParams& p, cudaStream_t stream) {
       return launch_mixed_mode<Mode::kMod>(p, stream);
     case Mode::kUpd:
       return launch_mixed_mode<Mode::kUpd>(p, stream);
+    case Mode::kCut:
+      return launch_mixed_mode<Mode::kCut>(p, stream);
     case Mode::kBlur:
       return launch_mixed_mode<Mode::kBlur>(p, stream);
     case Mode::kBlurMag:
@@ -36,6 +38,7 @@ void configure_mixed_passes() {
   configure_mixed_mode<Mode::kInv>();
   configure_mixed_mode<Mode::kMod>();
   configure_mixed_mode<Mode::kUpd>();
+  configure_mixed_mode<Mode::kCut>();
   configure_mixed_mode<Mode::kBlur>();
   configure_mixed_mode<Mode::kBlurMag>();
   configure_mixed_mode<Mode::kGrad>();

@@ -90,7 +90,8 @@ __device__ __forceinline__ int fast_div(int n, unsigned recip) {
 }
 
 constexpr bool two_transforms(Mode m) {
-  return m == Mode::kMod || m == Mode::kGrad || m == Mode::kUpd || m == Mode::kBlur ||
+  return m == Mode::kMod || m == Mode::kGrad || m == Mode::kUpd || m == Mode::kCut ||
+         m == Mode::kBlur ||
          m == Mode::kBlurMag;
 }
 
@@ -113,7 +114,8 @@ struct MixedSums {
 
 template <Mode M, bool ROWS>
 struct MixedPass {
-  static constexpr bool kFirstInverse = M == Mode::kInv || M == Mode::kUpd;
+  static constexpr bool kFirstInverse =
+      M == Mode::kInv || M == Mode::kUpd || M == Mode::kCut;
 
   const PassParams& p;
   const MixedShape& g;
@@ -186,7 +188,7 @@ struct MixedPass {
 #pragma unroll
         for (int q = 0; q < R; ++q) side.amp[q] = to_float(a[q * step]);
       }
-    } else if constexpr (M == Mode::kUpd) {
+    } else if constexpr (M == Mode::kUpd || M == Mode::kCut) {
 #pragma unroll
       for (int q = 0; q < R; ++q) side.outside |= (support[e + q * step] == 0 ? 1u : 0u) << q;
     }
@@ -221,6 +223,11 @@ struct MixedPass {
             x[e + q * step] = v[q];
           }
         }
+      }
+    } else if constexpr (M == Mode::kCut) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        if (side.outside >> q & 1u) v[q] = cscale(v[q], 0.0f);
       }
     } else if constexpr (M == Mode::kBlur || M == Mode::kBlurMag) {
       const float inv_l = 1.0f / static_cast<float>(p.L);
@@ -390,7 +397,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
         atomicAdd(&c->errs[static_cast<long long>(row) * p.starts_total + p.start0 + start], sum);
       }
     }
-  } else if constexpr (M == Mode::kUpd) {
+  } else if constexpr (M == Mode::kUpd || M == Mode::kCut) {
     if (p.bump_counter && blockIdx.x == 0 && threadIdx.x == 0) ++p.ctrl->counters[p.group];
   } else if constexpr (M == Mode::kBlur || M == Mode::kBlurMag) {
     if (p.level_method == 1) {

@@ -324,7 +324,9 @@ class Solver {
   // The latest error of every start (after at least one iteration of this run).
   std::vector<float> latest_errors();
   bool batched() const { return options_.variant != Variant::kPlain; }
-  bool wave_half() const { return wave_half_; }
+  // Graphs are kept by chunk length, kind of update and the wave's storage
+  // (the mixed variant switches it between stages).
+  int graph_key(int len) const { return 4 * len + (er_ ? 2 : 0) + (wave_half_ ? 1 : 0); }
   bool fp16_wave_variant() const {
     return options_.variant == Variant::kHalf || options_.variant == Variant::kMixed;
   }
@@ -356,7 +358,7 @@ class Solver {
   PassParams base(Mode mode, int axis3, int g) const;
 
   void load(const std::vector<ProblemView>& problems, std::uint64_t seed, const float2* start);
-  void enqueue_iteration(int g, cudaStream_t s);
+  void enqueue_iteration(int g, bool keep, cudaStream_t s);
   void enqueue_chunk(int len, cudaStream_t s);  // resident: `len` iterations in one launch
   // w = FFT_inner(x) for `count` starts from group g's first one
   void enqueue_establish(int g, int count);
@@ -421,7 +423,8 @@ class Solver {
   DeviceBuffer<double> errs_;
   int capacity_ = 0;
   bool wave_valid_ = false;
-  std::map<int, std::unique_ptr<Graph>> graphs_;  // by 2 * chunk length + wave_half_
+  bool er_ = false;  // the current stage is error reduction
+  std::map<int, std::unique_ptr<Graph>> graphs_;  // by graph_key()
   // Captured graphs run start groups as parallel branches, one stream each.
   std::vector<std::unique_ptr<Stream>> branches_;
   std::vector<cudaEvent_t> branch_events_;

@@ -1,0 +1,9 @@
+// Two-stage passes, mode kCut along rows: slice 0 of the lengths.
+
+#include "two_stage_kernel.cuh"
+
+namespace qpb {
+
+template TwoStageList two_stage_slice<Mode::kCut, true, 0>();
+
+}  // namespace qpb

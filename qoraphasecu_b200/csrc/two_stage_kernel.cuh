@@ -49,8 +49,9 @@ struct TwoStage {
   static constexpr int A = two_stage_large(L);
   static constexpr int B = L / A;
   static constexpr int T = A;  // threads of a line
-  static constexpr bool kTwo = M == Mode::kMod || M == Mode::kGrad || M == Mode::kUpd;
-  static constexpr bool kFirstInverse = M == Mode::kInv || M == Mode::kUpd;
+  static constexpr bool kTwo =
+      M == Mode::kMod || M == Mode::kGrad || M == Mode::kUpd || M == Mode::kCut;
+  static constexpr bool kFirstInverse = M == Mode::kInv || M == Mode::kUpd || M == Mode::kCut;
   static constexpr int kPitchA = A | 1;  // slots from thread to thread after the A-point stage
   static constexpr int kPitchB = B | 1;
   static constexpr int kUsed = std::max(B * kPitchA, kTwo ? A * kPitchB : 0);
@@ -128,7 +129,8 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
   }
   // what the point-wise step reads, in flight over the barrier
   [[maybe_unused]] float amp[M == Mode::kMod || M == Mode::kGrad ? B : 1];
-  [[maybe_unused]] unsigned char inside[M == Mode::kUpd ? B : 1];
+  constexpr bool kUpdate = M == Mode::kUpd || M == Mode::kCut;
+  [[maybe_unused]] unsigned char inside[kUpdate ? B : 1];
   [[maybe_unused]] float ca = p.coef_a, cb = p.coef_b;
   if constexpr (M == Mode::kMod || M == Mode::kGrad) {
     if (active) {
@@ -147,13 +149,13 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
         for (int q = 0; q < B; ++q) amp[q] = to_float(a[q * A * S]);
       }
     }
-  } else if constexpr (M == Mode::kUpd) {
+  } else if constexpr (kUpdate) {
     if (active) {
       const std::uint8_t* s = p.support + start_off + e;
 #pragma unroll
       for (int q = 0; q < B; ++q) inside[q] = s[q * A * S];
     }
-    if (p.coef_from_ctrl) {
+    if (M == Mode::kUpd && p.coef_from_ctrl) {
       ca = p.ctrl->a;
       cb = p.ctrl->b;
     }
@@ -193,6 +195,11 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
         if (!inside[q]) u[q] = relaxed(ca, xo, cb, u[q]);
         x[q * A * S] = u[q];
       }
+    } else if constexpr (M == Mode::kCut) {
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        if (!inside[q]) u[q] = cscale(u[q], 0.0f);
+      }
     } else {
 #pragma unroll
       for (int q = 0; q < B; ++q) u[q] = pointwise_projection<M>(u[q], amp[q], p.scale, error);
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
 #pragma unroll
     for (int q = 0; q < B; ++q) ex2[t * K::kPitchB + q] = u[q];
   }
-  if constexpr (M == Mode::kUpd) {
+  if constexpr (kUpdate) {
     if (p.bump_counter && blockIdx.x == 0 && tid == 0) ++p.ctrl->counters[p.group];
     __syncthreads();
   } else {

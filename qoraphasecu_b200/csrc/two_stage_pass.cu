@@ -30,6 +30,7 @@ const TwoStagePass* find(Mode mode, int L, bool rows) {
   if (rows) {
     switch (mode) {
       case Mode::kUpd: return table<Mode::kUpd, true>()[L];
+      case Mode::kCut: return table<Mode::kCut, true>()[L];
       case Mode::kFwdFromX: return table<Mode::kFwdFromX, true>()[L];
       case Mode::kInv: return table<Mode::kInv, true>()[L];
       default: return nullptr;
@@ -57,7 +58,7 @@ void launch_two_stage_pass(Mode mode, const PassParams& p, cudaStream_t stream) 
 }
 
 void configure_two_stage(int L) {
-  for (const Mode mode : {Mode::kUpd, Mode::kFwdFromX, Mode::kInv, Mode::kMod, Mode::kGrad,
+  for (const Mode mode : {Mode::kUpd, Mode::kCut, Mode::kFwdFromX, Mode::kInv, Mode::kMod, Mode::kGrad,
                           Mode::kFwd}) {
     for (const bool rows : {false, true}) {
       if (const TwoStagePass* pass = find(mode, L, rows)) pass->configure();
