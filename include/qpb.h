@@ -211,6 +211,12 @@ QPB_API qpb_status qpb_run(qpb_solver* solver, const qpb_op* ops, size_t n_ops);
 QPB_API qpb_status qpb_reset(qpb_solver* solver, const qpb_problem* problems, size_t n_problems,
                              uint64_t seed, const float* start);
 
+/* As qpb_reset, the given starts of every problem in an array of their own:
+ * starts[q] points to problem q's starts (no counterpart in the reference).
+ * They are copied straight from there, without one array of them all. */
+QPB_API qpb_status qpb_reset_starts(qpb_solver* solver, const qpb_problem* problems,
+                                    size_t n_problems, uint64_t seed, const float* const* starts);
+
 /* Bounded waits (no counterpart in the reference, whose kernels never wait on
  * one another). The line passes stage inputs by asynchronous bulk copies and
  * wait for them a bounded number of polls (about 4 million by default); a CTA

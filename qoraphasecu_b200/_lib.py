@@ -49,6 +49,7 @@ EXPORTS = (
     "qpb_create_device",
     "qpb_results_device",
     "qpb_reset",
+    "qpb_reset_starts",
     "qpb_run",
     "qpb_set_wait_limit",
     "qpb_set_progress",
@@ -151,6 +152,8 @@ def load():
         lib.qpb_results_device.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p]
         lib.qpb_run.argtypes = [c_void_p, POINTER(Op), c_size_t]
         lib.qpb_reset.argtypes = [c_void_p, POINTER(Problem), c_size_t, c_uint64, c_void_p]
+        lib.qpb_reset_starts.argtypes = [c_void_p, POINTER(Problem), c_size_t, c_uint64,
+                                         POINTER(c_void_p)]
         lib.qpb_set_progress.argtypes = [c_void_p, PROGRESS, c_void_p]
         lib.qpb_set_wait_limit.argtypes = [c_void_p, c_int, c_int]
         lib.qpb_error_count.argtypes = [c_void_p, POINTER(c_size_t)]

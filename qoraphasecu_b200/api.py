@@ -564,16 +564,18 @@ class BatchSolver:
             if tuple(new.shape) != tuple(old.shape):
                 raise ValueError(f"problem {q} has shape {tuple(new.shape)}, the batch was built "
                                  f"with {tuple(old.shape)}")
-        start = None
+        starts = None
         if init is not None:
             if len(init) != len(problems):
                 raise ValueError(f"init has {len(init)} entries for {len(problems)} problems")
-            start = np.concatenate([_start(i, p.shape, self._starts).ravel()
-                                    for i, p in zip(init, problems)])
+            starts = [_start(i, p.shape, self._starts) for i, p in zip(init, problems)]
         views = (_lib.Problem * len(problems))(*[p._c() for p in problems])
-        ptr = None if start is None else ctypes.c_void_p(start.ctypes.data)
-        _lib.check(self._lib.qpb_reset(self._handle, views, len(problems),
-                                       0 if seed is None else seed, ptr))
+        seed = 0 if seed is None else seed
+        if starts is None:
+            _lib.check(self._lib.qpb_reset(self._handle, views, len(problems), seed, None))
+        else:
+            each = (ctypes.c_void_p * len(starts))(*[a.ctypes.data for a in starts])
+            _lib.check(self._lib.qpb_reset_starts(self._handle, views, len(problems), seed, each))
         self.problems = problems
         self._views = views
 

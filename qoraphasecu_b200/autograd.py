@@ -21,6 +21,7 @@ a per-pixel magnitude bound.
 from __future__ import annotations
 
 import ctypes
+import math
 import time
 
 import numpy as np
@@ -72,8 +73,9 @@ def _loss_and_grad(x, signed, shape):
     if not x.is_cuda or x.dtype != torch.complex64:
         raise ValueError("x must be a complex64 CUDA tensor")
     x = x.contiguous()
-    batch = x.numel() // int(np.prod(shape))
-    if batch * int(np.prod(shape)) != x.numel():
+    numel = math.prod(shape)
+    batch = x.numel() // numel
+    if batch * numel != x.numel():
         raise ValueError(f"x of {x.numel()} elements is not a batch of {shape}")
     grad = torch.empty_like(x)
     loss = torch.empty(batch, dtype=torch.float64, device=x.device)

@@ -77,9 +77,7 @@ void amplitude_loss_grad(int ndim, const long long* shape, int batch, const floa
   const Dims3 d = dims_of(view);
   AdjointResources& r = resources();
   PassRunner runner(d, ndim, r.plans);
-  QPB_CHECK(cudaMemsetAsync(r.counter.get(), 0, sizeof(int), stream));
-  QPB_CHECK(cudaMemsetAsync(loss, 0, sizeof(double) * batch, stream));
-  set_ctrl(r.ctrl.get(), Ctrl{loss, 1, 0.0f, 0.0f, r.counter.get()}, stream);
+  begin_run(r.ctrl.get(), Ctrl{loss, 1, 0.0f, 0.0f, r.counter.get()}, 1, loss, batch, stream);
   auto params = [&](Mode m, int axis3) {
     PassParams p = runner.params(m, axis3, batch);
     p.w = grad;

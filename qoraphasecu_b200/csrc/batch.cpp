@@ -7,6 +7,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 #include "nvtx_range.hpp"
 
@@ -200,6 +201,18 @@ void BatchSolver::results(float2* objects, std::uint8_t* supports, float* errors
 
 void BatchSolver::reset(std::vector<ProblemView> problems, std::uint64_t seed,
                         const float2* start) {
+  std::vector<const float2*> starts;
+  if (start) {
+    for (const long long numel : numel_) {
+      starts.push_back(start);
+      start += spp_ * numel;
+    }
+  }
+  reset(std::move(problems), seed, starts);
+}
+
+void BatchSolver::reset(std::vector<ProblemView> problems, std::uint64_t seed,
+                        const std::vector<const float2*>& starts) {
   if (problems.size() != where_.size()) {
     throw InvalidArgument("reset needs as many problems as the batch was built with");
   }
@@ -209,27 +222,17 @@ void BatchSolver::reset(std::vector<ProblemView> problems, std::uint64_t seed,
       throw InvalidArgument("reset needs problem " + std::to_string(q) + " in its original shape");
     }
   }
-  if (classes_.size() == 1) {
-    classes_[0].solver->reset(problems, seed, start);
-    iteration_ = 0;
-    return;
-  }
-  if (start && on_device_) throw InvalidArgument("given starts on the device need problems of one shape");
-  std::vector<long long> start_off(problems.size(), 0);
-  for (std::size_t q = 1; q < problems.size(); ++q) {
-    start_off[q] = start_off[q - 1] + static_cast<long long>(spp_) * numel_[q - 1];
+  if (classes_.size() > 1 && !starts.empty() && on_device_) {
+    throw InvalidArgument("given starts on the device need problems of one shape");
   }
   for (Class& c : classes_) {
     std::vector<ProblemView> views;
-    std::vector<float2> given;
+    std::vector<const float2*> given;
     for (int q : c.members) {
       views.push_back(problems[q]);
-      if (start) {
-        const float2* src = start + start_off[q];
-        given.insert(given.end(), src, src + static_cast<std::size_t>(spp_) * numel_[q]);
-      }
+      if (!starts.empty()) given.push_back(starts[q]);
     }
-    c.solver->reset(views, seed, start ? given.data() : nullptr);
+    c.solver->reset(views, seed, given);
   }
   iteration_ = 0;
 }

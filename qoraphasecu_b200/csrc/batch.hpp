@@ -32,6 +32,9 @@ class BatchSolver {
   // q of problem q's shape at construction, host or device arrays as then),
   // new starts drawn from `seed` as a new batch would draw them, or given.
   void reset(std::vector<ProblemView> problems, std::uint64_t seed, const float2* start);
+  // `starts`: problem q's given starts, or empty.
+  void reset(std::vector<ProblemView> problems, std::uint64_t seed,
+             const std::vector<const float2*>& starts);
   bool on_device() const { return on_device_; }
   std::size_t error_count() const { return classes_[0].solver->error_count(); }
   int starts() const { return spp_ * static_cast<int>(where_.size()); }

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -142,13 +143,14 @@ qpb_status qpb_make_problem(const float* intensity, int ndim, const int64_t* sha
   return guarded([&] {
     const long long n = numel_checked(ndim, shape);
     require(intensity && amplitude_out && mask_out && support_out, "NULL array");
-    for (long long i = 0; i < n; ++i) {
-      if (!std::isfinite(intensity[i])) throw qpb::InvalidArgument("intensity contains NaN or Inf");
-    }
+    // whole-array reductions without an early exit, which the compiler vectorises
+    long long odd = 0;
+    for (long long i = 0; i < n; ++i) odd += !(std::fabs(intensity[i]) <= FLT_MAX);
+    if (odd) throw qpb::InvalidArgument("intensity contains NaN or Inf");
     if (mask) {
-      bool all_bad = true;
-      for (long long i = 0; i < n && all_bad; ++i) all_bad = mask[i] != 0;
-      if (all_bad) throw qpb::InvalidArgument("mask marks every pixel as bad; nothing left to fit");
+      long long usable = 0;
+      for (long long i = 0; i < n; ++i) usable += mask[i] == 0;
+      if (usable == 0) throw qpb::InvalidArgument("mask marks every pixel as bad; nothing left to fit");
     }
     long long sh[3] = {0, 0, 0};
     for (int a = 0; a < ndim; ++a) sh[a] = shape[a];
@@ -265,6 +267,24 @@ qpb_status qpb_reset(qpb_solver* solver, const qpb_problem* problems, size_t n_p
     for (size_t q = 0; q < n_problems; ++q) views.push_back(made_problem(problems + q));
     use_solver_device(solver);
     solver->impl.reset(views, seed, reinterpret_cast<const float2*>(start));
+  });
+}
+
+qpb_status qpb_reset_starts(qpb_solver* solver, const qpb_problem* problems, size_t n_problems,
+                            uint64_t seed, const float* const* starts) {
+  return guarded([&] {
+    require(solver != nullptr, "solver is NULL");
+    require(problems != nullptr && n_problems > 0, "no problems");
+    require(starts != nullptr, "starts is NULL");
+    std::vector<qpb::ProblemView> views;
+    std::vector<const float2*> given;
+    for (size_t q = 0; q < n_problems; ++q) {
+      views.push_back(made_problem(problems + q));
+      require(starts[q] != nullptr, "starts holds a NULL");
+      given.push_back(reinterpret_cast<const float2*>(starts[q]));
+    }
+    use_solver_device(solver);
+    solver->impl.reset(views, seed, given);
   });
 }
 

@@ -396,11 +396,24 @@ Solver::Solver(const std::vector<ProblemView>& problems, const SolverOptions& op
   };
   arena_ = DeviceBuffer<unsigned char>(lay_out(nullptr));
   lay_out(arena_.get());
-  load(problems, options.seed, options.start);
+  load(problems, options.seed, per_problem(options.start));
+}
+
+std::vector<const float2*> Solver::per_problem(const float2* start) const {
+  std::vector<const float2*> starts;
+  for (int q = 0; start && q < problems_; ++q) {
+    starts.push_back(start + static_cast<std::size_t>(q) * spp_ * n_);
+  }
+  return starts;
 }
 
 void Solver::reset(const std::vector<ProblemView>& problems, std::uint64_t seed,
                    const float2* start) {
+  reset(problems, seed, per_problem(start));
+}
+
+void Solver::reset(const std::vector<ProblemView>& problems, std::uint64_t seed,
+                   const std::vector<const float2*>& starts) {
   if (static_cast<int>(problems.size()) != problems_) {
     throw InvalidArgument("reset needs as many problems as the solver was built for");
   }
@@ -413,7 +426,7 @@ void Solver::reset(const std::vector<ProblemView>& problems, std::uint64_t seed,
       throw InvalidArgument("problem arrays do not match its shape; build it with make_problem");
     }
   }
-  load(problems, seed, start);
+  load(problems, seed, starts);
 }
 
 // Problems into the solver's buffers: per problem the FFT-order amplitude,
@@ -423,7 +436,8 @@ void Solver::reset(const std::vector<ProblemView>& problems, std::uint64_t seed,
 // arrays are staged there first); then the starts, drawn or given. The
 // captured graphs stay valid: every buffer keeps its address.
 void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
-                  const float2* start) {
+                  const std::vector<const float2*>& starts) {
+  const bool given = !starts.empty();
   PassParams mod = runner_.params(Mode::kMod, runner_.outer(), batch_);
   mod.amp_tiled = amp_tiled_;
   const int lines = amp_tiled_ == kAmpTiledLines     ? column_pass_lines(mod, Mode::kMod)
@@ -472,7 +486,7 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
     prepare_problem_device(
         v, d_, options_.amp_storage, mod.L, mod.S, lines, amp_tiled_ == kAmpTiledLines,
         // the FFT-order amplitude is what random starts are drawn on
-        start ? nullptr : amp_f_.get() + static_cast<std::size_t>(q) * n_,
+        given ? nullptr : amp_f_.get() + static_cast<std::size_t>(q) * n_,
         amp_.get() + static_cast<std::size_t>(q) * n_ * elem,
         support_.get() + static_cast<std::size_t>(q) * spp_ * n_, spp_,
         all_shares + static_cast<std::size_t>(q) * shares,
@@ -503,18 +517,26 @@ void Solver::load(const std::vector<ProblemView>& problems, std::uint64_t seed,
   const bool iter_half = iter_half_;
   wave_half_ = false;
   iter_half_ = false;
-  if (start) {
+  if (given) {
     // Given starts, centre-origin: to FFT order, cut to the support
     // (cpu_solver.cpp:37-41), brought into the scale of an fp16 variant's
     // amplitude (divided by its peak, as test_cuda.cpp:192-205 requires).
-    // Aligned starts in this device's memory are read where they are.
-    const float2* from = start;
-    cudaPointerAttributes where{};
-    QPB_CHECK(cudaPointerGetAttributes(&where, start));
-    if (where.type != cudaMemoryTypeDevice || where.device != select_.device ||
-        reinterpret_cast<std::uintptr_t>(start) % alignof(float2) != 0) {
-      QPB_CHECK(cudaMemcpyAsync(w_.get(), start, total * sizeof(float2), cudaMemcpyDefault,
-                                stream_));
+    // Aligned starts in this device's memory, one after another, are read
+    // where they are.
+    const std::size_t block = static_cast<std::size_t>(spp_) * n_;
+    const float2* from = starts[0];
+    bool in_place = reinterpret_cast<std::uintptr_t>(from) % alignof(float2) == 0;
+    for (std::size_t q = 0; q < starts.size(); ++q) in_place &= starts[q] == from + q * block;
+    if (in_place) {
+      cudaPointerAttributes where{};
+      QPB_CHECK(cudaPointerGetAttributes(&where, from));
+      in_place = where.type == cudaMemoryTypeDevice && where.device == select_.device;
+    }
+    if (!in_place) {
+      for (std::size_t q = 0; q < starts.size(); ++q) {
+        QPB_CHECK(cudaMemcpyAsync(w_.get() + q * block, starts[q], block * sizeof(float2),
+                                  cudaMemcpyDefault, stream_));
+      }
       from = w_.get();
     }
     roll_cut(from, support_.get(), x_.get(), d_, starts_,

@@ -278,7 +278,10 @@ class Solver {
   // New problems of the same shape and count in the same solver: buffers and
   // captured graphs are kept, the iterate, supports and error histories start
   // afresh from `seed` or the given starts (as construction does).
+  // The starts (null: drawn) come one array for all problems, or one for each.
   void reset(const std::vector<ProblemView>& problems, std::uint64_t seed, const float2* start);
+  void reset(const std::vector<ProblemView>& problems, std::uint64_t seed,
+             const std::vector<const float2*>& starts);
   std::size_t error_count() const { return errors_.empty() ? 0 : errors_[0].size(); }
   int starts() const { return starts_; }
   int problems() const { return problems_; }
@@ -357,7 +360,10 @@ class Solver {
   }
   PassParams base(Mode mode, int axis3, int g) const;
 
-  void load(const std::vector<ProblemView>& problems, std::uint64_t seed, const float2* start);
+  // `starts`: each problem's given starts, or empty.
+  void load(const std::vector<ProblemView>& problems, std::uint64_t seed,
+            const std::vector<const float2*>& starts);
+  std::vector<const float2*> per_problem(const float2* start) const;
   void enqueue_iteration(int g, bool keep, cudaStream_t s);
   void enqueue_chunk(int len, cudaStream_t s);  // resident: `len` iterations in one launch
   // w = FFT_inner(x) for `count` starts from group g's first one
