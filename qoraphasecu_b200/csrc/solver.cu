@@ -373,10 +373,15 @@ Solver::Solver(const std::vector<ProblemView>& problems, const SolverOptions& op
   const std::size_t elem = options.amp_storage == AmpStorage::kF32 ? 4 : 2;
   const std::size_t amps = static_cast<std::size_t>(problems_) * n_;
   const auto starts = static_cast<std::size_t>(starts_);
-  // Lays the buffers out from `base`; returns the bytes they take.
+  // Lays the large buffers out from `base` (and allocates the others with the
+  // second call); returns the bytes they take.
   auto lay_out = [&](unsigned char* base) {
     std::size_t at = 0;
     auto take = [&]<class T>(DeviceBuffer<T>& buffer, std::size_t count) {
+      if (count * sizeof(T) < kSmallAllocation) {
+        if (base) buffer = DeviceBuffer<T>(count);
+        return;
+      }
       if (base) buffer = DeviceBuffer<T>(reinterpret_cast<T*>(base + at), count);
       at += (count * sizeof(T) + 255) / 256 * 256;
     };
@@ -394,7 +399,7 @@ Solver::Solver(const std::vector<ProblemView>& problems, const SolverOptions& op
     take(counters_, static_cast<std::size_t>(groups_));
     return at;
   };
-  arena_ = DeviceBuffer<unsigned char>(lay_out(nullptr));
+  arena_ = DeviceBuffer<unsigned char>(std::max<std::size_t>(lay_out(nullptr), 256));
   lay_out(arena_.get());
   load(problems, options.seed, per_problem(options.start));
 }

@@ -401,8 +401,10 @@ class Solver {
   Stream stream_;
   PassRunner runner_;
   std::vector<double> energies_;     // usable energy per problem
-  // One allocation for the buffers below up to counters_ (an allocation of
-  // more than a megabyte costs about 0.35 ms, and as much to free).
+  // One allocation for the buffers below up to counters_ that are large: one
+  // of a megabyte or more costs about 0.35 ms and as much to free, a smaller
+  // one 3 us.
+  static constexpr std::size_t kSmallAllocation = 1 << 20;
   DeviceBuffer<unsigned char> arena_;
   long long amp_stride_ = 0;         // elements between problems' amplitudes in amp_
   DeviceBuffer<unsigned char> amp_;  // signed amplitude in the chosen storage
