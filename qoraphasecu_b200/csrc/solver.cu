@@ -854,11 +854,16 @@ void Solver::end_chunk(int len) {
   if (progress_ && iteration_ % options_.sync_every == 0) report();
 }
 
+// Iterations of one resident launch, at most.
+static constexpr int kResidentIterations = 1000;
+
 void Solver::iterate(int count, Coefficients c) {
   begin_iterate(c);
   for (int done = 0; done < count;) {
-    // the resident kernel runs a stage in one launch unless someone watches
-    const int len = resident_ && !progress_ ? count - done : chunk_length(count - done);
+    // the resident kernel runs a stage in one launch (some milliseconds at most)
+    // unless someone watches
+    const int len = resident_ && !progress_ ? std::min(count - done, kResidentIterations)
+                                            : chunk_length(count - done);
     if (resident_) {
       enqueue_chunk_body(len, stream_);
     } else if (batched()) {
