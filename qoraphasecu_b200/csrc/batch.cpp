@@ -9,7 +9,9 @@
 #include <string>
 #include <utility>
 
+#include "cluster_share.hpp"
 #include "nvtx_range.hpp"
+#include "resident.cuh"
 
 namespace qpb {
 
@@ -68,7 +70,33 @@ BatchSolver::BatchSolver(const std::vector<ProblemView>& problems, const SolverO
     events_.resize(classes_.size() + 1);
     for (auto& e : events_) QPB_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
+  share_sms();
   trace("batch: %zu problems in %zu shape classes", problems.size(), classes_.size());
+}
+
+// The resident classes run beside each other; each was given clusters as if it
+// had the device to itself.
+void BatchSolver::share_sms() {
+  std::vector<Solver*> resident;
+  std::vector<ClusterClaim> claims;
+  for (const Class& c : classes_) {
+    if (!c.solver->resident()) continue;
+    ClusterClaim claim{c.solver->side(), c.solver->starts(), {}};
+    for (const ClusterSize& s : cluster_sizes(claim.side)) {
+      claim.room.push_back(resident_max_clusters(claim.side, s.ctas));
+    }
+    resident.push_back(c.solver.get());
+    claims.push_back(std::move(claim));
+  }
+  if (resident.size() < 2) return;
+  int sms = 0;
+  QPB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, select_.device));
+  const std::vector<int> sizes = share_clusters(claims, sms);
+  for (std::size_t k = 0; k < resident.size(); ++k) {
+    resident[k]->set_cluster(sizes[k]);
+    trace("batch: %d starts of side %d in clusters of %d", claims[k].starts, claims[k].side,
+          sizes[k]);
+  }
 }
 
 BatchSolver::~BatchSolver() {

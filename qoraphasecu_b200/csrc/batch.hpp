@@ -59,6 +59,7 @@ class BatchSolver {
     std::unique_ptr<Solver> solver;
   };
   void report(int iteration);
+  void share_sms();
 
   DeviceSelect select_;
   Stream stream_;

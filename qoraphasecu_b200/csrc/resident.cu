@@ -51,6 +51,7 @@
 #include <vector>
 
 #include "bulk_copy.cuh"
+#include "cluster_share.hpp"
 #include "line_fft.cuh"
 #include "projection.cuh"
 #include "reduce.cuh"
@@ -345,16 +346,6 @@ void allow() {
   }
 }
 
-// Cluster sizes of a side, smallest first.
-std::vector<int> cluster_sizes(int side) {
-  switch (side) {
-    case 64: return {1, 2, 4, 8};
-    case 128: return {2, 4, 8, 16};
-    case 256: return {8, 16};
-    default: return {};
-  }
-}
-
 // Clusters of each size that the current device runs at once, the attributes
 // set on the way; once per device and side.
 const std::map<int, int>& cluster_room(int side) {
@@ -367,7 +358,8 @@ const std::map<int, int>& cluster_room(int side) {
   if (fresh) {
     try {
       with_side(side, [&](auto n) {
-        for (const int size : cluster_sizes(n)) {
+        for (const ClusterSize& s : cluster_sizes(n)) {
+          const int size = s.ctas;
           with_cluster<n>(size, [&](auto c) {
             allow<n, c, float>();
             allow<n, c, __half>();
@@ -392,7 +384,7 @@ const std::map<int, int>& cluster_room(int side) {
 
 int resident_max_clusters(int side, int cluster) { return cluster_room(side).at(cluster); }
 
-int resident_smallest_cluster(int side) { return cluster_sizes(side).front(); }
+int resident_smallest_cluster(int side) { return cluster_sizes(side).front().ctas; }
 
 bool resident_supports(int ndim, int d1, int d2) {
   return ndim == 2 && d1 == d2 && (d1 == 64 || d1 == 128 || d1 == 256);

@@ -286,6 +286,9 @@ class Solver {
   int starts() const { return starts_; }
   int problems() const { return problems_; }
   bool resident() const { return resident_; }
+  int side() const { return d_.d2; }
+  // The resident schedule's CTAs per start; before anything is captured.
+  void set_cluster(int cluster) { cluster_ = cluster; }
   bool persistent() const { return persistent_; }
   int batch() const { return batch_; }
   long long numel() const { return n_; }
