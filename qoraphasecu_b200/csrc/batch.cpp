@@ -21,6 +21,7 @@ BatchSolver::BatchSolver(const std::vector<ProblemView>& problems, const SolverO
       spp_(options.starts),
       every_(options.sync_every),
       batched_(options.variant != Variant::kPlain),
+      mixed_(options.variant == Variant::kMixed),
       on_device_(!problems.empty() && problems[0].on_device) {
   if (problems.empty()) throw InvalidArgument("no problems");
   if (options.starts < 1) throw InvalidArgument("starts must be >= 1");
@@ -135,6 +136,14 @@ void BatchSolver::run(const OpDesc* ops, std::size_t count) {
   validate_recipe(ops, count);
   const NvtxRange recipe_range("batch recipe", recipe_iterations(ops, count));
   for (Class& c : classes_) c.solver->begin_run(ops, count);
+  graphs_.plan(ops, count, classes_[0].solver->iteration(), every_, !mixed_);
+  IterationCost cost;
+  for (const Class& c : classes_) {
+    const IterationCost of = c.solver->iteration_cost();
+    cost.passes += of.passes;
+    cost.us += of.us;
+    cost.saved_us += of.saved_us;
+  }
   for (std::size_t i = 0; i < count; ++i) {
     const OpDesc& o = ops[i];
     const NvtxRange stage_range(op_name(o.kind), o.n);
@@ -157,9 +166,13 @@ void BatchSolver::run(const OpDesc* ops, std::size_t count) {
     for (int done = 0; done < o.n;) {
       const int len = classes_[0].solver->chunk_length(o.n - done);
       if (batched_) {
-        const int key = classes_[0].solver->graph_key(len);
-        auto it = graphs_.find(key);
-        if (it == graphs_.end()) {
+        const bool half = classes_[0].solver->wave_half();
+        const bool cut = o.kind == kOpER &&
+                         graphs_.cut(len, half, (o.n - done) / len, cost,
+                                     classes_[0].solver->run_iterations());
+        for (Class& c : classes_) c.solver->set_cut(cut);
+        const Graph* graph = graphs_.find(len, cut, half);
+        if (!graph) {
           for (Class& c : classes_) c.solver->prepare_branches();
           const unsigned long long before = launches();
           QPB_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -178,15 +191,18 @@ void BatchSolver::run(const OpDesc* ops, std::size_t count) {
             if (broken) cudaGraphDestroy(broken);
             throw;
           }
-          cudaGraph_t graph{};
-          QPB_CHECK(cudaStreamEndCapture(stream_, &graph));
+          cudaGraph_t captured{};
+          QPB_CHECK(cudaStreamEndCapture(stream_, &captured));
           const unsigned long long kernels = launches() - before;
           count_launches(0ULL - kernels);  // counted again on every replay
-          it = graphs_.emplace(key, std::make_unique<Graph>(graph, kernels)).first;
+          graph = &graphs_.add(len, cut, half, captured, kernels);
         }
-        it->second->launch(stream_);
+        graph->launch(stream_);
       } else {
-        for (Class& c : classes_) c.solver->enqueue_chunk_body(len, stream_);
+        for (Class& c : classes_) {
+          c.solver->set_cut(o.kind == kOpER);
+          c.solver->enqueue_chunk_body(len, stream_);
+        }
       }
       for (Class& c : classes_) c.solver->end_chunk(len);
       iteration_ += len;

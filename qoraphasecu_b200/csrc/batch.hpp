@@ -4,13 +4,12 @@
 // is one Solver over all its problems (one batched launch per pass or resident
 // chunk for all of them, its schedule picked by the autotuner for that shape
 // and start count). Every chunk of iterations of every class is captured into
-// ONE graph per chunk length: the classes are parallel branches of it, so the
+// ONE graph per chunk length and kind (ChunkGraphs): the classes are parallel branches of it, so the
 // small problems fill the SMs the large ones leave idle. Shrinkwrap and detwin
 // run between chunks, as in a single solver. A batch of one problem is exactly
 // a Solver.
 #pragma once
 
-#include <map>
 #include <memory>
 #include <vector>
 
@@ -66,13 +65,14 @@ class BatchSolver {
   int spp_;
   int every_;
   bool batched_;  // chunks captured into graphs (else launched directly)
+  bool mixed_;
   bool on_device_;  // problem arrays given as device pointers
   std::vector<Class> classes_;
   std::vector<std::pair<int, int>> where_;  // problem -> (class, index in class)
   std::vector<long long> numel_;            // per problem
   std::vector<std::unique_ptr<Stream>> branches_;  // one per class
   std::vector<cudaEvent_t> events_;                // fork + one join per class
-  std::map<int, std::unique_ptr<Graph>> graphs_;   // by chunk length
+  ChunkGraphs graphs_;
   ProgressFn progress_ = nullptr;
   void* progress_user_ = nullptr;
   int iteration_ = 0;

@@ -218,6 +218,54 @@ int recipe_iterations(const OpDesc* ops, std::size_t count) {
   return static_cast<int>(total);
 }
 
+// ----------------------------------------------------------------- ChunkGraphs
+namespace {
+// Capture, instantiation and first launch of a graph, us of host time a kernel
+// node: 160 nodes in 8 branches take 75 + 600 + 260 us, 20 in one branch 100.
+// Making a second graph in the first pass of a new solver (20 RAAR and 80 ER
+// iterations) against replaying the first: 32 starts of 256 x 256 in 8 groups
+// 3270 and 2870 us, 16 of 240 x 240 in 8 groups 3220 and 2830, in one group,
+// where the making hides behind the RAAR stage, 1680 and 1800.
+constexpr double kNodeUs = 5.5;
+}  // namespace
+
+void ChunkGraphs::plan(const OpDesc* ops, std::size_t count, int iteration, int every,
+                       bool one_wave) {
+  feedback_.clear();
+  for (std::size_t i = 0; i < count; ++i) {
+    const bool feedback = ops[i].kind == kOpHIO || ops[i].kind == kOpRAAR;
+    if (!feedback && ops[i].kind != kOpER) continue;
+    for (int done = 0; done < ops[i].n;) {
+      const int len = std::min(ops[i].n - done, every - iteration % every);
+      if (feedback && one_wave) feedback_.insert(len);
+      iteration += len;
+      done += len;
+    }
+  }
+}
+
+bool ChunkGraphs::cut(int len, bool half, int chunks, const IterationCost& cost, int queued) {
+  if (cost.saved_us <= 0.0) return false;
+  if (find(len, true, half)) return true;
+  if (!find(len, false, half) && !feedback_.contains(len)) return true;
+  int& shared = shared_[len];
+  const double making = kNodeUs * cost.passes * len - cost.us * queued;
+  if ((shared + chunks) * cost.saved_us * len >= making) return true;
+  ++shared;
+  return false;
+}
+
+const Graph* ChunkGraphs::find(int len, bool cut, bool half) const {
+  const auto it = graphs_.find(key(len, cut, half));
+  return it == graphs_.end() ? nullptr : it->second.get();
+}
+
+const Graph& ChunkGraphs::add(int len, bool cut, bool half, cudaGraph_t graph,
+                              unsigned long long kernels) {
+  auto made = std::make_unique<Graph>(graph, kernels);
+  return *(graphs_[key(len, cut, half)] = std::move(made));
+}
+
 // ------------------------------------------------------------------ PassRunner
 PassRunner::PassRunner(Dims3 d, int ndim, PlanCache& plans)
     : d_(d), ndim_(ndim), wait_failures_(plans.wait_failures()), wait_tries_(kMaxWaitTries) {
@@ -695,6 +743,7 @@ void Solver::begin_run(const OpDesc* ops, std::size_t count) {
   qpb::begin_run(ctrl_.get(), Ctrl{errs_.get(), capacity_, 0.0f, 0.0f, counters_.get()}, groups_,
                  errs_.get(), static_cast<long long>(needed), stream_);
   run_iterations_ = 0;
+  graphs_.plan(ops, count, iteration_, options_.sync_every, options_.variant != Variant::kMixed);
 }
 
 void Solver::apply(const OpDesc& o) {
@@ -837,15 +886,29 @@ void Solver::enqueue_chunk_body(int len, cudaStream_t s) {
     for (int g = 0; g < groups_; ++g) {
       cudaStream_t b = *branches_[g];
       QPB_CHECK(cudaStreamWaitEvent(b, branch_events_[0], 0));
-      for (int i = 0; i < len; ++i) enqueue_iteration(g, !er_ || i == len - 1, b);
+      for (int i = 0; i < len; ++i) enqueue_iteration(g, !cut_ || i == len - 1, b);
       QPB_CHECK(cudaEventRecord(branch_events_[g + 1], b));
       QPB_CHECK(cudaStreamWaitEvent(s, branch_events_[g + 1], 0));
     }
   } else {
     for (int g = 0; g < groups_; ++g) {
-      for (int i = 0; i < len; ++i) enqueue_iteration(g, !er_ || i == len - 1, s);
+      for (int i = 0; i < len; ++i) enqueue_iteration(g, !cut_ || i == len - 1, s);
     }
   }
+}
+
+// Time: two dependent launches take 9 us however small, large arrays 53 bytes an
+// element (85 in 3D) at 7 TB/s. Saved: a read and a write of the iterate (8
+// bytes an element, 4 in fp16) at 15 TB/s, between the 7 measured for 4 starts
+// of 128^3, beyond L2, and the 25 for 32 of 256 x 256, in L2.
+IterationCost Solver::iteration_cost() const {
+  if (resident_ || persistent_) return {};
+  const double elements = static_cast<double>(n_) * starts_;
+  IterationCost c;
+  c.passes = groups_ * (runner_.has_mid() ? 4 : 2);
+  c.us = std::max(9.0, (runner_.has_mid() ? 85.0 : 53.0) * elements / 7e6);
+  c.saved_us = (iter_half_ ? 8.0 : 16.0) * elements / 15e6;
+  return c;
 }
 
 void Solver::end_chunk(int len) {
@@ -867,10 +930,11 @@ void Solver::iterate(int count, Coefficients c) {
     if (resident_) {
       enqueue_chunk_body(len, stream_);
     } else if (batched()) {
-      const int key = graph_key(len);
-      auto it = graphs_.find(key);
-      trace("iterate chunk len=%d graph=%s", len, it == graphs_.end() ? "capture" : "cached");
-      if (it == graphs_.end()) {
+      cut_ = er_ && graphs_.cut(len, wave_half_, (count - done) / len, iteration_cost(),
+                                run_iterations_);
+      const Graph* graph = graphs_.find(len, cut_, wave_half_);
+      trace("iterate chunk len=%d cut=%d graph=%s", len, cut_, graph ? "cached" : "capture");
+      if (!graph) {
         prepare_branches();
         const unsigned long long before = launches();
         QPB_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -882,14 +946,15 @@ void Solver::iterate(int count, Coefficients c) {
           if (broken) cudaGraphDestroy(broken);
           throw;
         }
-        cudaGraph_t graph{};
-        QPB_CHECK(cudaStreamEndCapture(stream_, &graph));
+        cudaGraph_t captured{};
+        QPB_CHECK(cudaStreamEndCapture(stream_, &captured));
         const unsigned long long kernels = launches() - before;
         count_launches(0ULL - kernels);  // counted again on every replay
-        it = graphs_.emplace(key, std::make_unique<Graph>(graph, kernels)).first;
+        graph = &graphs_.add(len, cut_, wave_half_, captured, kernels);
       }
-      it->second->launch(stream_);
+      graph->launch(stream_);
     } else {
+      cut_ = er_;
       enqueue_chunk_body(len, stream_);
     }
     end_chunk(len);

@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -207,6 +208,45 @@ struct OpDesc {
   int axis;
 };
 
+// One iteration as its chunks' graphs hold it: the passes it launches, an
+// estimate of the time they take, and what error reduction saves of it by
+// leaving the iterate alone (0 where one kernel runs a chunk), in us.
+struct IterationCost {
+  int passes = 0;
+  double us = 0.0;
+  double saved_us = 0.0;
+};
+
+// The captured graphs of a run's chunks, by chunk length, whether the updates
+// leave the iterate alone (error reduction, Mode::kCut) and the wave's storage
+// (the mixed variant switches it between stages).
+class ChunkGraphs {
+ public:
+  // Notes the chunk lengths at which the recipe's HIO and RAAR stages need a
+  // graph, its chunks ending at multiples of `every` iterations. `one_wave`:
+  // ER runs on the same wave storage, so it could replay theirs.
+  void plan(const OpDesc* ops, std::size_t count, int iteration, int every, bool one_wave);
+  // Whether the next error-reduction chunk, one of `chunks` of `len` iterations
+  // to come, leaves the iterate alone. It does unless it can replay a HIO or
+  // RAAR stage's graph (the same results, the iterate written in every
+  // iteration) and making a graph of its own would keep the device waiting for
+  // longer than it has saved and is about to; the `queued` iterations enqueued
+  // before it in this run hide a part of that. So a solver of many groups that
+  // runs one recipe makes one graph a length, one that is kept ends up with both.
+  bool cut(int len, bool half, int chunks, const IterationCost& cost, int queued);
+  // The graph of such a chunk, null before add().
+  const Graph* find(int len, bool cut, bool half) const;
+  const Graph& add(int len, bool cut, bool half, cudaGraph_t graph, unsigned long long kernels);
+  void clear() { graphs_.clear(); }
+
+ private:
+  static int key(int len, bool cut, bool half) { return 4 * len + (cut ? 2 : 0) + (half ? 1 : 0); }
+
+  std::map<int, std::unique_ptr<Graph>> graphs_;
+  std::set<int> feedback_;     // chunk lengths of this run's HIO and RAAR stages
+  std::map<int, int> shared_;  // error-reduction chunks run on their graphs, by length
+};
+
 using ProgressFn = void (*)(void* user, int iteration, const float* errors, int count);
 
 // Throws Timeout when a line pass planned from `plans` gave up a bounded wait
@@ -330,9 +370,11 @@ class Solver {
   // The latest error of every start (after at least one iteration of this run).
   std::vector<float> latest_errors();
   bool batched() const { return options_.variant != Variant::kPlain; }
-  // Graphs are kept by chunk length, kind of update and the wave's storage
-  // (the mixed variant switches it between stages).
-  int graph_key(int len) const { return 4 * len + (er_ ? 2 : 0) + (wave_half_ ? 1 : 0); }
+  bool wave_half() const { return wave_half_; }
+  IterationCost iteration_cost() const;
+  void set_cut(bool cut) { cut_ = cut; }  // for the next chunk
+  int iteration() const { return iteration_; }
+  int run_iterations() const { return run_iterations_; }
   bool fp16_wave_variant() const {
     return options_.variant == Variant::kHalf || options_.variant == Variant::kMixed;
   }
@@ -434,8 +476,9 @@ class Solver {
   DeviceBuffer<double> errs_;
   int capacity_ = 0;
   bool wave_valid_ = false;
-  bool er_ = false;  // the current stage is error reduction
-  std::map<int, std::unique_ptr<Graph>> graphs_;  // by graph_key()
+  bool er_ = false;   // the current stage is error reduction
+  bool cut_ = false;  // the current chunk's updates leave the iterate alone
+  ChunkGraphs graphs_;
   // Captured graphs run start groups as parallel branches, one stream each.
   std::vector<std::unique_ptr<Stream>> branches_;
   std::vector<cudaEvent_t> branch_events_;
