@@ -56,6 +56,7 @@ BatchSolver::BatchSolver(const std::vector<ProblemView>& problems, const SolverO
     SolverOptions o = options;
     o.stream = stream_;
     o.device = select_.device;
+    o.chunked = classes_.size() > 1;
     std::vector<float2> given;
     if (options.start && classes_.size() > 1) {
       for (int q : c.members) {

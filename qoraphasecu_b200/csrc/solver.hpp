@@ -177,6 +177,7 @@ struct SolverOptions {
   cudaStream_t stream = nullptr;    // work stream lent by the caller; null = own stream
   bool tune = true;                 // batch == 0: let the autotuner pick starts per launch
   Schedule schedule = Schedule::kAuto;
+  bool chunked = false;  // part of a batch, which runs every stage in chunks of sync_every
 };
 
 // The schedule the autotuner picks for this problem and start count: the

@@ -32,8 +32,9 @@ namespace qpb {
 namespace {
 
 // device, d0, d1, d2, starts, amplitude storage, resident kernel among the
-// candidates, variant (fp16 storage changes the passes' cost)
-using Key = std::tuple<int, int, int, int, int, int, bool, int>;
+// candidates, variant (fp16 storage changes the passes' cost), chunked stages
+// (a resident launch then ends with each chunk)
+using Key = std::tuple<int, int, int, int, int, int, bool, int, bool>;
 
 std::mutex g_mutex;
 std::map<Key, TunedSchedule> g_choice;
@@ -61,16 +62,20 @@ double time_candidate(const ProblemView& problem, const SolverOptions& base, int
   o.stream = nullptr;
   // The caller's chunk length (10..100 iterations), so that each candidate
   // replays the graphs the caller's run would replay; two chunks per timing
-  // keep the host's share of the wall time small.
+  // keep the host's share of the wall time small. The resident kernel runs
+  // them in one launch, as in the caller's run, or in one each where the
+  // caller's stages are chunked: two stages then.
   o.sync_every = std::max(10, std::min(base.sync_every, 100));
   o.variant = base.variant == Variant::kPlain ? Variant::kBatched : base.variant;
   Solver solver(problem, o);
-  const OpDesc raar{kOpRAAR, 2 * o.sync_every, 0.9f, 0.0f, 0.0f, 0, 0};
-  solver.run(&raar, 1);  // captures the graph
+  const std::size_t stages = base.chunked ? 2 : 1;
+  const OpDesc raar{kOpRAAR, o.sync_every * (base.chunked ? 1 : 2), 0.9f, 0.0f, 0.0f, 0, 0};
+  const OpDesc recipe[2] = {raar, raar};
+  solver.run(recipe, stages);  // captures the graph
   double best = 1e30;
   for (int rep = 0; rep < 3; ++rep) {
     const auto t0 = std::chrono::steady_clock::now();
-    solver.run(&raar, 1);
+    solver.run(recipe, stages);
     const auto t1 = std::chrono::steady_clock::now();
     best = std::min(best, std::chrono::duration<double>(t1 - t0).count());
   }
@@ -87,7 +92,7 @@ TunedSchedule tuned_schedule(const ProblemView& problem, const SolverOptions& op
   int device = 0;
   QPB_CHECK(cudaGetDevice(&device));
   const Key key{device, d.d0, d.d1, d.d2, starts, static_cast<int>(options.amp_storage),
-                resident_ok, static_cast<int>(options.variant)};
+                resident_ok, static_cast<int>(options.variant), options.chunked};
   std::lock_guard<std::mutex> lock(g_mutex);
   if (auto it = g_choice.find(key); it != g_choice.end()) return it->second;
   std::vector<int> candidates;
@@ -134,13 +139,13 @@ std::string tuning_report() {
   std::lock_guard<std::mutex> lock(g_mutex);
   std::ostringstream out;
   for (const auto& [key, choice] : g_choice) {
-    const auto& [device, d0, d1, d2, starts, storage, resident_ok, variant] = key;
+    const auto& [device, d0, d1, d2, starts, storage, resident_ok, variant, chunked] = key;
     out << "device " << device << " shape " << d0 << "x" << d1 << "x" << d2 << " starts "
         << starts << " storage " << storage
         << (variant == static_cast<int>(Variant::kHalf)    ? " half"
             : variant == static_cast<int>(Variant::kMixed) ? " mixed"
                                                            : "")
-        << ": "
+        << (chunked ? " in a batch" : "") << ": "
         << (choice.resident     ? std::string("resident")
             : choice.persistent ? std::string("persistent")
                                 : "batch " + std::to_string(choice.batch))
