@@ -917,15 +917,21 @@ void Solver::end_chunk(int len) {
   if (progress_ && iteration_ % options_.sync_every == 0) report();
 }
 
-// Iterations of one resident launch, at most.
-static constexpr int kResidentIterations = 1000;
+// Iterations of one resident launch, at most: 1000 where all starts are resident
+// at once, fewer by the waves they run in otherwise, so that a launch ends after
+// 2 (64 x 64) to 12 ms (256 x 256) whatever the number of starts.
+int Solver::resident_iterations() const {
+  const int room = std::max(1, resident_max_clusters(d_.d2, cluster_));
+  const int waves = (starts_ + room - 1) / room;
+  return std::max(1, 1000 / waves);
+}
 
 void Solver::iterate(int count, Coefficients c) {
   begin_iterate(c);
   for (int done = 0; done < count;) {
-    // the resident kernel runs a stage in one launch (some milliseconds at most)
+    // the resident kernel runs a stage in one launch, if it is not too long,
     // unless someone watches
-    const int len = resident_ && !progress_ ? std::min(count - done, kResidentIterations)
+    const int len = resident_ && !progress_ ? std::min(count - done, resident_iterations())
                                             : chunk_length(count - done);
     if (resident_) {
       enqueue_chunk_body(len, stream_);

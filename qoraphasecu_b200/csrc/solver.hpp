@@ -411,6 +411,7 @@ class Solver {
             const std::vector<const float2*>& starts);
   std::vector<const float2*> per_problem(const float2* start) const;
   void enqueue_iteration(int g, bool keep, cudaStream_t s);
+  int resident_iterations() const;
   void enqueue_chunk(int len, cudaStream_t s);  // resident: `len` iterations in one launch
   // w = FFT_inner(x) for `count` starts from group g's first one
   void enqueue_establish(int g, int count);
