@@ -5,11 +5,18 @@
 // which lets its CTAs start while the kernel before it in the stream (the
 // previous pass) runs its last CTAs: launch, scheduling and the shared-memory
 // set-up overlap that kernel's tail instead of following it. Every CTA then
-// waits, before its first access of global memory, until the kernel before it
-// has completed and its writes are visible, and lets the kernel after it
-// start early in turn. Both instructions are no-ops when the kernel was
-// launched without the attribute or follows no kernel; the waits end when
-// the kernel before ends, so nothing here waits on a condition of its own.
+// waits, before its first access of memory that the kernel before it may have
+// written, until that kernel has completed and its writes are visible, and only
+// then lets the kernel after it start early in turn. Both instructions are
+// no-ops when the kernel was launched without the attribute or follows no
+// kernel; the waits end when the kernel before ends, so nothing here waits on a
+// condition of its own.
+//
+// So what was written ahead of the kernel before is there from a CTA's start:
+// the two-stage passes read the amplitude and the support before their wait.
+// Those have writers of their own (the problem set-up, shrinkwrap's threshold,
+// detwin), plain launches or copies, and none of them may be what a pass
+// directly follows: Solver::begin_iterate enqueues a kernel ahead of every stage.
 #pragma once
 
 #include <cuda_runtime.h>

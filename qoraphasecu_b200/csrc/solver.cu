@@ -851,6 +851,8 @@ void Solver::begin_iterate(Coefficients c) {
     }
   }
   if (!wave_valid_) establish_wave();
+  // also the kernel between a writer of the support (shrinkwrap, detwin) and
+  // the stage's passes, which may read it ahead of their wait
   set_coefficients(ctrl_.get(), c.a, c.b, stream_);
 }
 

@@ -114,9 +114,10 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
   float2* ex = smem + l * K::kLine;
   float2* side = smem + lpc * K::kLine;  // second exchange, or the old iterate
 
-  // What the point-wise step reads besides the arrays of the iteration: no
-  // pass writes it, so the loads are issued before the wait for the pass
-  // before (an iteration of 4 starts of 96 x 96 5.8 -> 5.3 us, of 16 of
+  // What the point-wise step reads besides the arrays of the iteration: its
+  // writers (problem set-up, threshold, detwin) are never the kernel right
+  // before a pass (dependent_launch.cuh), so the loads are issued before the
+  // wait for that one (an iteration of 4 starts of 96 x 96 5.8 -> 5.3 us, of 16 of
   // 240 x 240 15.5 -> 14.5).
   [[maybe_unused]] float amp[M == Mode::kMod || M == Mode::kGrad ? B : 1];
   constexpr bool kUpdate = M == Mode::kUpd || M == Mode::kCut;
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(TwoStage<L, M, ROWS>::kThreads, TwoStage<L, M,
       for (int q = 0; q < B; ++q) inside[q] = s[q * A * S];
     }
   }
-  wait_for_prior_kernel();  // the wave, the iterate, the support and the control block
+  wait_for_prior_kernel();  // the wave, the iterate and the control block
   allow_next_kernel();
 
   if constexpr (M == Mode::kUpd) {
