@@ -73,6 +73,10 @@ def _configure(lib):
     return lib
 
 
+class LibraryMissing(FileNotFoundError):
+    """The reference's compiled code is not there (its sources are needed to build it)."""
+
+
 def load_variant(which: str):
     """One of the oracle libraries: "cpu" (the reference's CPU path), "cuda"
     (plus the reference's own CUDA backend) or "dropin" (the reference's core
@@ -80,7 +84,7 @@ def load_variant(which: str):
     path = {"cpu": LIBRARY, "cuda": CUDA_LIBRARY, "dropin": DROPIN_LIBRARY}[which]
     if which not in _libs:
         if not path.exists():
-            raise FileNotFoundError(f"{path} is missing: build it with oracle/Makefile")
+            raise LibraryMissing(f"{path.name} is missing: build it with oracle/Makefile")
         _libs[which] = _configure(ctypes.CDLL(str(path)))
     return _libs[which]
 
