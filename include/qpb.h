@@ -59,8 +59,10 @@ typedef enum qpb_variant {
 /* How BATCHED iterations run (no counterpart in the reference). STREAMED: two
  * line passes per 2D iteration (four in 3D) through HBM, start groups as
  * parallel graph branches. RESIDENT: square 2D problems of side 64, 128 or 256
- * only; each start's iterate stays in the shared memory of a thread-block
- * cluster for a whole chunk of sync_every iterations, one launch per chunk.
+ * only; each start stays on chip, in the registers and shared memory of a
+ * thread-block cluster, for a whole launch: a stage (long ones in several
+ * launches), or sync_every iterations where progress is reported or a batch of
+ * several shapes runs.
  * PERSISTENT: 2D problems with sides of 64, 128 or 256 (complex64 storage);
  * a chunk of sync_every iterations of every start is one launch whose CTAs
  * claim the passes' tiles from a work list, each tile waiting (bounded) only

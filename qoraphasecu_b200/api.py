@@ -734,7 +734,7 @@ def reconstruct(
         progress: ``fn(iteration, errors)`` every ``sync_every`` iterations.
         schedule: how batched iterations run: ``"streamed"`` line passes,
             ``"resident"`` (square 2D of side 64, 128 or 256: each start held in
-            a thread-block cluster's shared memory), ``"persistent"`` (2D with
+            a thread-block cluster's registers and shared memory), ``"persistent"`` (2D with
             sides of 64, 128 or 256: a chunk of iterations of every start as
             one launch walking a work list of tiles) or ``"auto"`` (timed once
             per shape and start count).

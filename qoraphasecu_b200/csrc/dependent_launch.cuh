@@ -35,7 +35,7 @@ __device__ __forceinline__ void wait_for_prior_kernel() {
 }
 
 // Allows the kernel after this one to be scheduled (it still waits for this
-// kernel's completion before touching memory).
+// kernel's completion before touching what this one may write).
 __device__ __forceinline__ void allow_next_kernel() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

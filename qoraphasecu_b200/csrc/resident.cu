@@ -401,8 +401,6 @@ int resident_cluster(int side, int starts) {
   return best;
 }
 
-void configure_resident(int side) { cluster_room(side); }
-
 void launch_resident(const ResidentParams& p, int side, int starts, cudaStream_t stream) {
   if (p.iterations < 1) return;
   with_side(side, [&](auto n) {

@@ -1,6 +1,7 @@
 // Resident iteration kernel: whole iterations of square 2D problems (side 64,
-// 128 or 256) with each start's iterate, wave and support held in the shared
-// memory of a thread-block cluster for a whole chunk of iterations.
+// 128 or 256) with each start held by a thread-block cluster for a whole launch,
+// iterate, support and amplitudes in registers, the lines that its CTAs
+// exchange in shared memory.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,7 +36,8 @@ bool resident_supports(int ndim, int d1, int d2);
 // CTAs per start (the cluster size) for `starts` starts of side N on the
 // current device: the largest size at which every start is resident at once
 // with one CTA per SM, else the smallest. More SMs per start shorten an
-// iteration's serial chain as long as they would be idle otherwise.
+// iteration's serial chain as long as they would be idle otherwise (classes of
+// a batch run beside each other: cluster_share.hpp).
 int resident_cluster(int side, int starts);
 
 // Clusters of that size of the side-N kernel that the current device runs at once.
@@ -47,9 +49,5 @@ void launch_resident(const ResidentParams& p, int side, int starts, cudaStream_t
 
 // The smallest cluster a start of side N fits.
 int resident_smallest_cluster(int side);
-
-// Sets the attributes of side N's kernels on the current device (once per
-// device, outside stream capture; resident_cluster does so too).
-void configure_resident(int side);
 
 }  // namespace qpb

@@ -161,7 +161,7 @@ enum class Variant : int {
 enum class Schedule : int {
   kAuto = 0,      // the autotuner picks (streamed groups, resident or persistent)
   kStreamed = 1,  // two (3D: four) streamed line passes per iteration, start groups as branches
-  kResident = 2,  // one resident-cluster launch per chunk of iterations (square 2D, side 64/128/256)
+  kResident = 2,  // resident-cluster launches, a stage or a chunk each (square 2D, side 64/128/256)
   kPersistent = 3,  // one work-list launch per chunk of iterations (2D, sides 64/128/256)
 };
 

@@ -3,8 +3,8 @@
 //
 // Starts are independent, so any schedule gives the same iterates; what
 // changes is how the work fills the GPU. The resident kernel keeps each start
-// in a cluster's shared memory for a whole chunk of iterations, but one start
-// takes up to 8 SMs, so few starts leave SMs idle. With streamed passes, one
+// in the registers and shared memory of a cluster, but a cluster runs one start
+// at a time and its SMs wait at its barriers. With streamed passes, one
 // group of all starts is a single chain of kernels per iteration whose last
 // CTAs run with the SMs half idle; several smaller groups become parallel
 // branches of the captured graph, and one group's modulus pass then overlaps
