@@ -68,10 +68,18 @@ struct TwoStage {
   // spares them a barrier; one transform needs one.
   static constexpr int kSideSlots = M == Mode::kUpd ? L : (kTwo ? kLine : 0);
   // Amplitudes read before the wait for the pass before hold B registers over
-  // the A-point DFT: a gain where A is at most 16 (240: 7.8 -> 7.5 us), a loss
-  // above (300: 4.8 -> 5.6 us).
+  // the A-point DFT. Measured at 21 lengths of 45 to 625, launches of 300 k and
+  // of 2 M elements, early against late: with A at most 16 the small launches
+  // gain 4 to 7% (5 starts of 240: 4.77 -> 4.44 us; nothing at 144 and 150, -3%
+  // at 100) and the large ones 0 to 3%, with A = 18, 20 and 24 both lose 7 to
+  // 22% (2 of 360: 5.2 -> 6.3 us); at A = 21 and 25 it is within 6% either way.
   static constexpr bool kEarlyAmplitude = A <= 16;
   // Registers: about 2 A + 48 a thread for the larger DFT and its addresses.
+  // At the same lengths a step less (64, 80, 104) costs the modulus pass of the
+  // small launches 5 to 18% with A at most 16 and up to 32% above (of the large
+  // ones -4 to 24%), a step more (104, 128, 168) that of the large launches 0 to
+  // 23%; small ones gain 4 to 7% from it at 100, 144, 600 and 625 alone. The
+  // updates are indifferent (5% at most).
   static constexpr int kRegisters = A <= 10 ? 80 : (A <= 16 ? 104 : 128);
   static constexpr int kBlocks = std::max(1, std::min(16, 65536 / (kThreads * kRegisters)));
 };
