@@ -232,6 +232,7 @@ constexpr double kNodeUs = 5.5;
 void ChunkGraphs::plan(const OpDesc* ops, std::size_t count, int iteration, int every,
                        bool one_wave) {
   feedback_.clear();
+  started_.reset();
   for (std::size_t i = 0; i < count; ++i) {
     const bool feedback = ops[i].kind == kOpHIO || ops[i].kind == kOpRAAR;
     if (!feedback && ops[i].kind != kOpER) continue;
@@ -249,8 +250,13 @@ bool ChunkGraphs::cut(int len, bool half, int chunks, const IterationCost& cost,
   if (find(len, true, half)) return true;
   if (!find(len, false, half) && !feedback_.contains(len)) return true;
   int& shared = shared_[len];
-  const double making = kNodeUs * cost.passes * len - cost.us * queued;
-  if ((shared + chunks) * cost.saved_us * len >= making) return true;
+  double waiting = kNodeUs * cost.passes * len;
+  if (started_) {
+    const std::chrono::duration<double, std::micro> since =
+        std::chrono::steady_clock::now() - *started_;
+    waiting -= std::max(0.0, cost.us * queued - since.count());
+  }
+  if ((shared + chunks) * cost.saved_us * len >= waiting) return true;
   ++shared;
   return false;
 }
@@ -264,6 +270,11 @@ const Graph& ChunkGraphs::add(int len, bool cut, bool half, cudaGraph_t graph,
                               unsigned long long kernels) {
   auto made = std::make_unique<Graph>(graph, kernels);
   return *(graphs_[key(len, cut, half)] = std::move(made));
+}
+
+void ChunkGraphs::launch(const Graph& graph, cudaStream_t stream) {
+  graph.launch(stream);
+  if (!started_) started_ = std::chrono::steady_clock::now();
 }
 
 // ------------------------------------------------------------------ PassRunner
@@ -960,7 +971,7 @@ void Solver::iterate(int count, Coefficients c) {
         count_launches(0ULL - kernels);  // counted again on every replay
         graph = &graphs_.add(len, cut_, wave_half_, captured, kernels);
       }
-      graph->launch(stream_);
+      graphs_.launch(*graph, stream_);
     } else {
       cut_ = er_;
       enqueue_chunk_body(len, stream_);

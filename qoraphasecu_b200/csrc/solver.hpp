@@ -8,9 +8,11 @@
 
 #include <cuda_runtime.h>
 
+#include <chrono>
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <optional>
 #include <set>
 #include <string>
 #include <vector>
@@ -231,13 +233,15 @@ class ChunkGraphs {
   // to come, leaves the iterate alone. It does unless it can replay a HIO or
   // RAAR stage's graph (the same results, the iterate written in every
   // iteration) and making a graph of its own would keep the device waiting for
-  // longer than it has saved and is about to; the `queued` iterations enqueued
-  // before it in this run hide a part of that. So a solver of many groups that
-  // runs one recipe makes one graph a length, one that is kept ends up with both.
+  // longer than it has saved and is about to; what the device has still to do of
+  // the `queued` iterations enqueued before it in this run hides a part of that.
+  // So a solver of many groups that runs one recipe makes one graph a length, one
+  // that is kept ends up with both.
   bool cut(int len, bool half, int chunks, const IterationCost& cost, int queued);
   // The graph of such a chunk, null before add().
   const Graph* find(int len, bool cut, bool half) const;
   const Graph& add(int len, bool cut, bool half, cudaGraph_t graph, unsigned long long kernels);
+  void launch(const Graph& graph, cudaStream_t stream);
   void clear() { graphs_.clear(); }
 
  private:
@@ -246,6 +250,7 @@ class ChunkGraphs {
   std::map<int, std::unique_ptr<Graph>> graphs_;
   std::set<int> feedback_;     // chunk lengths of this run's HIO and RAAR stages
   std::map<int, int> shared_;  // error-reduction chunks run on their graphs, by length
+  std::optional<std::chrono::steady_clock::time_point> started_;  // this run's first launch
 };
 
 using ProgressFn = void (*)(void* user, int iteration, const float* errors, int count);

@@ -50,7 +50,7 @@ def test_error_reduction_alone_has_its_own(gpu):
 
 
 def test_a_kept_solver_ends_up_with_both(gpu):
-    runs = captures((240, 240), 16, 2, ", ".join(["Recipe(RAAR(20), ER(30))"] * 22))
+    runs = captures((240, 240), 16, 2, ", ".join(["Recipe(RAAR(20), ER(30))"] * 40))
     assert runs[0] == 1 and sum(runs) == 2 and runs[-1] == 0
 
 
